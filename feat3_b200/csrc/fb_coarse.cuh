@@ -14,6 +14,7 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include "fb_dense.cuh"
 #include "fb_mf.cuh"
 
 namespace fb {
@@ -36,7 +37,8 @@ struct CoarseArgs {
   CLevel<T> L[kCoarseMax];  // L[0] = first fused level, L[nlv-1] = coarsest
   int nlv, nu, coarse;
   T omega;
-  const T* cinv;            // dense inverse of the coarsest filtered system (FB_COARSE_DIRECT)
+  const T* cinv;            // dense operator of the last level (FB_COARSE_DIRECT), rows of ldc
+  uint32_t ldc;
   int s1_coarsest;          // the restriction onto the coarsest level forms its first smoothing step
 };
 
@@ -200,6 +202,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_coarse_cycle(CoarseArgs<T> A) {
   cgr::cluster_group cl = cgr::this_cluster();
   __shared__ double sh[THREADS / 32];
   __shared__ double part[2][16];  // cluster partials, double-buffered
+  __shared__ __align__(16) T sb[kDenseRows];  // right-hand side of the last level's dense product
   const uint32_t gt = cl.block_rank() * THREADS + threadIdx.x;
   const uint32_t gs = cl.num_blocks() * THREADS;
   const int nu = A.nu;
@@ -257,13 +260,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_coarse_cycle(CoarseArgs<T> A) {
     const CLevel<T>& L = A.L[l];
     const T* b = L.rhs;
     if (A.coarse == FB_COARSE_DIRECT) {
-      const uint32_t lane = gt & 31;
-      for (uint32_t row = gt >> 5; row < L.n; row += gs >> 5) {
-        double s = 0.0;
-        for (uint32_t j = lane; j < L.n; j += 32) s += double(__ldg(A.cinv + uint64_t(row) * L.n + j)) * double(ldc(b + j));
-        s = warp_sum(s);
-        if (lane == 0) L.x[row] = T(s);
-      }
+      for (uint32_t i = threadIdx.x; i < A.ldc; i += THREADS) sb[i] = i < L.n ? ldc(b + i) : T(0);
+      __syncthreads();
+      dense_rows(A.cinv, A.ldc, sb, L.n, gt >> 5, gs >> 5, gt & 31, [&](uint32_t row, double s) { L.x[row] = T(s); });
       cl.sync();
       sol[l] = L.x;
     } else if (A.coarse == FB_COARSE_SMOOTHER) {

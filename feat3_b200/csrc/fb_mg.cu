@@ -21,6 +21,7 @@
 #include "fb_stencil_stream.cuh"
 #include "fb_rest_staged.cuh"
 #include "fb_coarse.cuh"
+#include "fb_dense.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -239,19 +240,6 @@ template<typename T>
 __global__ void k_skip_fix(T* out, const T* __restrict__ s0, const double* skip_src, uint32_t n) {
   if (!smoother_skip<T>(skip_src)) return;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = s0[i];
-}
-
-// dense coarse solve: x = Cinv b (Cinv = inverse of the filtered coarse matrix, zero
-// Dirichlet rows/columns); one warp per row
-template<typename T>
-__global__ void k_dense_solve(T* x, const T* __restrict__ cinv, const T* __restrict__ b, uint32_t n) {
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= n) return;
-  double s = 0.0;
-  for (uint32_t j = lane; j < n; j += 32) s += double(cinv[uint64_t(warp) * n + j]) * double(b[j]);
-  s = warp_sum(s);
-  if (lane == 0) x[warp] = T(s);
 }
 
 // coarse "none": x = filter_cor(b)
@@ -1016,6 +1004,71 @@ static int presmooth(fb_mg* m, int l, const T* b, const double* bnorm, bool need
   return FB_OK;
 }
 
+// ------------------------------------------------------------------ dense small end
+// The V-cycle's last level and its solver: the level of the dense operator when one was built
+// (build_dense), else the coarsest level with the configured coarse solver.
+static int last_level(const fb_mg* m) { return m->dense_l > 0 ? m->dense_l : (int)m->L.size() - 1; }
+static int last_solver(const fb_mg* m) { return m->dense_l > 0 ? FB_COARSE_DIRECT : m->cfg.coarse; }
+
+template<typename T>
+static int launch_dense(fb_mg* m, int l, const T* b) {
+  Level& L = m->L[l];
+  const bool op = l == m->dense_l;
+  const T* a;
+  if constexpr (std::is_same<T, double>::value) a = op ? m->dop64 : m->cinv64; else a = op ? m->dop32 : m->cinv32;
+  const uint32_t ld = dense_ld(L.n);
+  k_dense_solve<T><<<grid_for(L.n, 4 * kDenseR), 128, ld * sizeof(T), m->stream>>>(Prec<T>::x(L), a, ld, b, L.n);
+  m->launches++;
+  FB_CHECK_LAUNCH();
+  return FB_OK;
+}
+
+// Forms the dense operator of the small end (V-cycle with the fixed coarse-grid correction, a linear
+// coarse solver): the first level below the finest with at most kDenseRows rows, when it is not the
+// coarsest one already.
+template<typename T, int NC>
+static int launch_dense_build(fb_mg* m, const DenseArgs& D, T* op, size_t smem) {
+  auto fn = k_dense_build<T, NC>;
+  FB_CUDA(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  const uint32_t n = D.L[0].n;
+  fn<<<(n + NC - 1) / NC, kDenseThreads, smem, m->stream>>>(D, op, dense_ld(n));
+  FB_CHECK_LAUNCH();
+  return FB_OK;
+}
+
+template<typename T>
+static int build_dense(fb_mg* m, T** op) {
+  const int nl = (int)m->L.size();
+  m->dense_l = 0;
+  if (m->cfg.cycle != FB_CYCLE_V || m->cfg.adapt_cgc != FB_CGC_FIXED || m->cfg.coarse == FB_COARSE_PCG) return FB_OK;
+  int ld = 1;
+  while (ld < nl && m->L[ld].n > kDenseRows) ++ld;
+  if (ld >= nl - 1 || nl - ld > kDenseMax) return FB_OK;
+  DenseArgs D{};
+  D.nlv = nl - ld; D.nu = m->cfg.nu; D.coarse = m->cfg.coarse; D.omega = m->cfg.omega_rich;
+  D.cinv = m->cinv64; D.ldc = dense_ld(m->L[nl - 1].n);
+  uint64_t rows = 0;
+  for (int i = 0; i < D.nlv; ++i) {
+    Level& L = m->L[ld + i];
+    if (!L.A.v64 || (i + 1 < D.nlv && (!L.P.v64 || !L.R.v64))) return FB_OK;
+    D.L[i].n = L.n; D.L[i].A = L.A.view(FB_PREC_F64); D.L[i].mask = L.mask; D.L[i].invd = L.invd64;
+    if (i + 1 < D.nlv) { D.L[i].P = L.P.view(false); D.L[i].R = L.R.view(false); }
+    rows += L.n;
+  }
+  // NC unit vectors per CTA: as many of 4, 2, 1 as the level vectors leave room for
+  const size_t per = size_t(rows) * 3 * sizeof(double), cap = 220 * 1024;
+  if (per > cap) return FB_OK;
+  const uint32_t n = m->L[ld].n;
+  const uint64_t size = uint64_t(n) * dense_ld(n);
+  if (!*op && dalloc(m, op, size) != FB_OK) return FB_OK;  // no room: level by level
+  FB_CUDA(cudaMemsetAsync(*op, 0, sizeof(T) * size, m->stream));
+  if (4 * per <= cap) FB_TRY((launch_dense_build<T, 4>(m, D, *op, 4 * per)));
+  else if (2 * per <= cap) FB_TRY((launch_dense_build<T, 2>(m, D, *op, 2 * per)));
+  else FB_TRY((launch_dense_build<T, 1>(m, D, *op, per)));
+  m->dense_l = ld;
+  return FB_OK;
+}
+
 // ------------------------------------------------------------------ fused coarse cycle
 // levels up to this size go to the one-cluster kernel: 3D level 4 (4,913 rows) and below. The
 // 3D level 5 (35,937 rows) runs faster as separate full-GPU launches (measured: 19.8 vs 20.3 ms
@@ -1054,7 +1107,7 @@ static int coarse_cluster_size(fb_mg* m) {
 // first level of the fused coarse cycle, or nl when the coarse end runs level by level
 template<typename T>
 static int coarse_start(fb_mg* m) {
-  const int nl = (int)m->L.size();
+  const int nl = last_level(m) + 1;
   if (m->cfg.format != FB_FORMAT_MATFREE || m->cfg.coarse == FB_COARSE_PCG || (m->cfg.flags & FB_FLAG_NO_COARSE_FUSION))
     return nl;
   int lc = nl;
@@ -1063,20 +1116,23 @@ static int coarse_start(fb_mg* m) {
     lc = l;
   }
   if (nl - lc < 2 || nl - lc > kCoarseMax) return nl;
+  if (last_solver(m) == FB_COARSE_DIRECT && m->L[nl - 1].n > kDenseRows) return nl;
   const int cs = m->dim == 3 ? coarse_cluster_size<T, 3>(m) : coarse_cluster_size<T, 2>(m);
   return cs > 0 ? lc : nl;
 }
 
 template<typename T>
 static int launch_coarse(fb_mg* m, int lc, T** sol_lc) {
-  const int nl = (int)m->L.size();
+  const int nl = last_level(m) + 1;
   CoarseArgs<T> A;
   A.nlv = nl - lc;
   A.nu = m->cfg.nu;
-  A.coarse = m->cfg.coarse;
+  A.coarse = last_solver(m);
   A.omega = T(m->cfg.omega_rich);
-  if constexpr (std::is_same<T, double>::value) A.cinv = m->cinv64; else A.cinv = m->cinv32;
-  A.s1_coarsest = m->cfg.coarse == FB_COARSE_SMOOTHER ? 1 : 0;
+  const bool op = m->dense_l > 0;
+  if constexpr (std::is_same<T, double>::value) A.cinv = op ? m->dop64 : m->cinv64; else A.cinv = op ? m->dop32 : m->cinv32;
+  A.ldc = dense_ld(m->L[nl - 1].n);
+  A.s1_coarsest = A.coarse == FB_COARSE_SMOOTHER ? 1 : 0;
   for (int i = 0; i < A.nlv; ++i) {
     Level& L = m->L[lc + i];
     CLevel<T>& c = A.L[i];
@@ -1120,7 +1176,7 @@ static int launch_coarse(fb_mg* m, int lc, T** sol_lc) {
 
 template<typename T>
 static int vcycle(fb_mg* m, const T* rhs_top, const double* rhs_top_sumsq, T** out_top) {
-  const int nl = (int)m->L.size();
+  const int nl = last_level(m) + 1, coarse = last_solver(m);
   const int nu = m->cfg.nu;
   const T omega = T(m->cfg.omega_rich);
   std::vector<T*> sol(nl, nullptr);
@@ -1137,7 +1193,7 @@ static int vcycle(fb_mg* m, const T* rhs_top, const double* rhs_top_sumsq, T** o
     FB_TRY(spmv_L<T>(m, L, sol[l], ed, nullptr));
     const bool coarsest_next = (l + 2 == nl);
     T* s1 = nullptr;
-    if (nu >= 2 && (!coarsest_next || m->cfg.coarse == FB_COARSE_SMOOTHER)) s1 = Prec<T>::x(C);
+    if (nu >= 2 && (!coarsest_next || coarse == FB_COARSE_SMOOTHER)) s1 = Prec<T>::x(C);
     EpiRestrict<T> er{Prec<T>::rhs(C), s1, Prec<T>::invd(C), C.mask, omega};
     FB_TRY(rest_T<T>(m, l, Prec<T>::def(L), er, &m->sc->lvl[2 * (l + 1)]));
   }
@@ -1149,13 +1205,9 @@ static int vcycle(fb_mg* m, const T* rhs_top, const double* rhs_top_sumsq, T** o
     Level& L = m->L[l];
     const T* b = (l == 0) ? rhs_top : Prec<T>::rhs(L);
     const double* bn = (l == 0) ? rhs_top_sumsq : &m->sc->lvl[2 * l];
-    switch (m->cfg.coarse) {
+    switch (coarse) {
       case FB_COARSE_DIRECT: {
-        const T* cinv;
-        if constexpr (std::is_same<T, double>::value) cinv = m->cinv64; else cinv = m->cinv32;
-        k_dense_solve<T><<<grid_for(uint64_t(L.n) * 32, 256), 256, 0, m->stream>>>(Prec<T>::x(L), cinv, b, L.n);
-        m->launches++;
-        FB_CHECK_LAUNCH();
+        FB_TRY(launch_dense<T>(m, l, b));
         sol[l] = Prec<T>::x(L);
         break;
       }
@@ -1290,11 +1342,7 @@ struct Cycle {
     const T* b = rhs(l);
     switch (m->cfg.coarse) {
       case FB_COARSE_DIRECT: {
-        const T* cinv;
-        if constexpr (std::is_same<T, double>::value) cinv = m->cinv64; else cinv = m->cinv32;
-        k_dense_solve<T><<<grid_for(uint64_t(L.n) * 32, 256), 256, 0, m->stream>>>(Prec<T>::x(L), cinv, b, L.n);
-        m->launches++;
-        FB_CHECK_LAUNCH();
+        FB_TRY(launch_dense<T>(m, l, b));
         sol[l] = Prec<T>::x(L);
         break;
       }
@@ -1663,10 +1711,12 @@ static int ensure_vectors(fb_mg* m, int prec) {
     }
   }
   if (low && m->cinv64 && !m->cinv32) {
-    FB_TRY(dalloc(m, &m->cinv32, uint64_t(m->nc) * m->nc));
-    k_cvt<float, double><<<ew_grid(uint64_t(m->nc) * m->nc), 256, 0, m->stream>>>(m->cinv32, m->cinv64, uint64_t(m->nc) * m->nc);
+    const uint64_t size = uint64_t(m->nc) * dense_ld(m->nc);
+    FB_TRY(dalloc(m, &m->cinv32, size));
+    k_cvt<float, double><<<ew_grid(size), 256, 0, m->stream>>>(m->cinv32, m->cinv64, size);
     FB_CHECK_LAUNCH();
   }
+  FB_TRY(low ? build_dense<float>(m, &m->dop32) : build_dense<double>(m, &m->dop64));
   const uint32_t n = m->L[0].n;
   if (!m->r) {
     FB_TRY(dalloc(m, &m->r, n)); FB_TRY(dalloc(m, &m->p, n)); FB_TRY(dalloc(m, &m->q, n));
@@ -1795,7 +1845,10 @@ int build_coarse_inverse(fb_mg* m, const HostCsr& A, const std::vector<uint32_t>
     for (uint64_t j = 0; j < n; ++j)
       if (dir[i] || dir[j]) inv[i * n + j] = 0.0;
   m->nc = uint32_t(n);
-  FB_TRY(dupload(m, &m->cinv64, inv.data(), inv.size()));
+  const uint64_t ld = dense_ld(uint32_t(n));
+  std::vector<double> rows(n * ld, 0.0);
+  for (uint64_t i = 0; i < n; ++i) std::copy(inv.begin() + i * n, inv.begin() + (i + 1) * n, rows.begin() + i * ld);
+  FB_TRY(dupload(m, &m->cinv64, rows.data(), rows.size()));
   return FB_OK;
 }
 

@@ -136,7 +136,11 @@ struct fb_mg {
   // coarse direct solver
   uint32_t nc = 0;
   double* cinv64 = nullptr;
-  float* cinv32 = nullptr;
+  float* cinv32 = nullptr;       // (rows of dense_ld(nc))
+  // the small end of the V-cycle as a dense operator (fb_dense.cuh): its level, 0 = none
+  int dense_l = 0;
+  double* dop64 = nullptr;
+  float* dop32 = nullptr;
   // outer (finest) vectors
   double *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *xb = nullptr, *bb = nullptr;
   float* p32 = nullptr;          // FP32 search direction of the mixed matrix-free form
@@ -208,6 +212,8 @@ int upload_filter(fb_mg* m, Level& L, const std::vector<uint32_t>& f);
 // feat_io: rhs and sol are in the C-ABI's numbering (FEAT order when m->feat_dof is set)
 int solve_dev(fb_mg* m, const double* rhs, double* sol, double* hist, fb_solve_info* info, bool feat_io = true);
 unsigned ew_grid(uint64_t n);
+// row length of a stored dense operator (16-byte rows in FP32 and FP64)
+inline uint32_t dense_ld(uint32_t n) { return (n + 3u) & ~3u; }
 int feat_numbering(int dim, int degree, int level, uint32_t* dof_lex, uint32_t* cell_lex, cudaStream_t s);
 // dst[perm[i]] = src[i] (FEAT order -> lattice order) and dst[i] = src[perm[i]] (back)
 int perm_to_lattice(fb_mg* m, double* dst, const double* src, const uint32_t* perm, uint64_t n);

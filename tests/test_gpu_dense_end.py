@@ -1,0 +1,67 @@
+"""The small end of the V-cycle as one dense operator: one cycle against the oracle's, whose coarse
+levels run step by step, for the smoothing counts, coarse solvers and element types the operator is
+formed for, on hierarchies whose first level of at most 1,280 rows has one to five levels below it."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+# dim, degree, level, level_min, nu, coarse
+CASES = [(2, 1, 6, 1, 1, "none"), (2, 1, 7, 2, 3, "smoother"), (2, 1, 6, 4, 2, "direct"), (3, 1, 5, 1, 2, "direct"),
+         (3, 1, 4, 0, 2, "smoother"), (2, 2, 5, 1, 4, "direct"), (3, 2, 3, 1, 2, "none")]
+
+
+def relerr(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def coefficient(dim, level):
+    return np.exp(np.random.default_rng(5).standard_normal((1 << level) ** dim))
+
+
+@pytest.mark.parametrize("case", CASES, ids=["d%dq%dL%d-%d-nu%d-%s" % c for c in CASES])
+@pytest.mark.parametrize("fmt", ["sell", "stencil", "matfree"])
+def test_cycle_matches_oracle(case, fmt):
+    from feat3_b200.solver import MultiGrid
+    dim, deg, lvl, lmin, nu, coarse = case
+    k = coefficient(dim, lvl)
+    H = po.Hierarchy(dim, deg, lvl, lmin, k)
+    d = H.rhs("one") * np.random.default_rng(6).uniform(0.5, 1.5, H.ndofs())
+    ref = H.vcycle(d, nu=nu, coarse=coarse)
+    mg = MultiGrid.structured(dim, deg, lvl, lmin, k)
+    dd = torch.tensor(d).cuda()
+    first = None
+    # FP64 to rounding; FP32 within 100 roundings of 2^-24 (some 50 dependent steps)
+    for prec, tol in (("f64", 1e-13), ("f32", 6e-6), ("f64", 1e-13)):
+        mg.configure(nu=nu, coarse=coarse, precision=prec, format=fmt)
+        out = mg.vcycle(dd).cpu().numpy()
+        assert relerr(out, ref) <= tol, prec
+        if prec == "f64":
+            first = out if first is None else first
+            np.testing.assert_array_equal(out, first)
+    # the other cycles do not use the operator; the V-cycle after them does again
+    mg.configure(nu=nu, coarse=coarse, format=fmt, cycle="w")
+    mg.vcycle(dd)
+    mg.configure(nu=nu, coarse=coarse, format=fmt)
+    np.testing.assert_array_equal(mg.vcycle(dd).cpu().numpy(), first)
+    assert not mg.vcycle(torch.zeros_like(dd)).any()
+    mg.close()
+
+
+@pytest.mark.parametrize("sigma", [1, 32])
+def test_handed_hierarchy_matches_oracle(sigma):
+    from feat3_b200.solver import MultiGrid
+    H = po.Hierarchy(2, 2, 5, 1, coefficient(2, 5))
+    levels = []
+    for l in range(5, 0, -1):
+        e = {"A": H.csr(l), "filter": H.filter(l)}
+        if l > 1:
+            e["P"], e["R"] = H.prol(l), H.rest(l)
+        levels.append(e)
+    d = H.rhs("one")
+    mg = MultiGrid.from_csr(levels, sell_sigma=sigma).configure(nu=3)
+    assert relerr(mg.vcycle(torch.tensor(d).cuda()).cpu().numpy(), H.vcycle(d, nu=3)) <= 1e-13
+    mg.close()
