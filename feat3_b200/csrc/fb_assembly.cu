@@ -801,8 +801,9 @@ int fb_mg_export_csr(fb_mg* m, int l, uint64_t* rp, uint32_t* col, double* val) 
     const uint32_t lr = feat.empty() ? r : feat[r];
     const uint32_t sr = slot_of[lr], c = sr / 32, t = sr % 32;
     row.clear();
-    for (uint32_t j = 0; j < rl[lr]; ++j) {
-      const uint32_t cl = cc[cs[c] + uint64_t(j) * 32 + t];
+    for (uint64_t j = 0; row.size() < rl[lr]; ++j) {
+      const uint32_t cl = cc[cs[c] + j * 32 + t];
+      if (cl == 0xffffffffu) continue;  // an empty slot of a chunk that follows a pattern
       row.emplace_back(feat.empty() ? cl : lat_to_feat[cl], vv[cs[c] + uint64_t(j) * 32 + t]);
     }
     if (!feat.empty()) std::sort(row.begin(), row.end(), [](const std::pair<uint32_t, double>& a, const std::pair<uint32_t, double>& b) { return a.first < b.first; });

@@ -52,13 +52,14 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseArgs D, T* o
       p += 3 * s;
     }
   }
-  // A x at a slot row (the thread's column of the NC)
+  // A x at a slot row (the thread's column of the NC); empty slots carry column ~0u
   auto product = [&](const DLevel& L, const double* x, uint32_t sr, uint32_t c) {
     const uint32_t ch = sr >> 5, e = L.A.cs[ch] + (sr & 31u), len = L.A.cl[ch];
     const double* val = static_cast<const double*>(L.A.val);
     double s = 0.0;
     for (uint32_t j = 0; j < len; ++j) {
-      s += __ldg(val + e + j * 32u) * x[size_t(__ldg(L.A.col + e + j * 32u)) * NC + c];
+      const uint32_t cc = __ldg(L.A.col + e + j * 32u);
+      if (cc != 0xffffffffu) s += __ldg(val + e + j * 32u) * x[size_t(cc) * NC + c];
     }
     return s;
   };

@@ -83,14 +83,10 @@ static void debug_check_ptrs(const char* what, std::initializer_list<const void*
 
 template<typename VT, typename XT, typename AT, typename Epi>
 static int launch_sell(fb_mg* m, const DevSell& A, int prec, const XT* x, const Epi& epi, double* red_out) {
-  // 2-byte values are read two slots per load from their interleaved layout (k_quant16_sell): 534
-  // against 579 us per FP16 Jacobi step at 257^3 with one 2-byte load per slot and 32 slots in
-  // flight per lane (602 us with 16, 624 us with 8); unrolling the pair loop 2 or 4 times ran 814-817
-  // us. Their odd last slot, if any, takes the slot loop below the pair loop.
-  auto fn = k_sell<VT, XT, AT, Epi, 8>;
+  auto fn = k_sell<VT, XT, AT, Epi>;
   const int grid = occupancy_grid((const void*)fn, A.nchunks);
   if (debug_enabled())
-    debug_check_ptrs("k_sell", {A.cs, A.cl, A.col, A.view(prec).val, (const void*)x, (const void*)m->ws,
+    debug_check_ptrs("k_sell", {A.cs, A.md, A.col, A.view(prec).val, (const void*)x, (const void*)m->ws,
                                 (const void*)m->counter, (const void*)red_out, (const void*)A.perm});
   fn<<<grid, 256, 0, m->stream>>>(A.view(prec), x, epi, m->ws, m->counter, red_out);
   m->launches++;
@@ -1617,10 +1613,168 @@ static int run_body(fb_mg* m, int j) {
   return FB_OK;
 }
 
+// ------------------------------------------------------------------ setup: offset patterns of a SELL matrix
+// A chunk follows a pattern when lane r's column in slot j is (slot row of r) + offset[j]: a row
+// with an entry in every slot (the reference lane) sets the offsets, and every other row's entries
+// follow them in the same order, with gaps (a lattice row next to the boundary, a Q2 edge row
+// between vertex rows). The row's entries move to the slots they match and the gaps hold value 0
+// (column ~0u in the 32-bit array, the mark of an empty slot). Every slot row + offset is a valid
+// column for all 32 lanes. The products and their order are those of the plain form (plus 0 * x of a
+// neighbouring column in the gaps).
+struct SellSetup {
+  uint32_t rows, cols, nchunks;
+  const uint32_t *cs, *cl, *rl, *perm;
+  uint32_t* col;
+  double* val;
+  uint32_t* md;
+  int32_t* pat;     // kSellPatterns x kSellPatternSlots
+  uint32_t* plen;   // slots of each pattern (0 = none)
+};
+
+// pass 0: md = length | (1 + reference lane) << 23 for chunks that could follow a pattern, else 0
+__global__ void __launch_bounds__(256) k_sell_candidates(SellSetup S) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < S.nchunks; c += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t e0 = S.cs[c], len = S.cl[c], sr = c * 32u + lane;
+    const uint32_t mylen = sr < S.rows ? S.rl[S.perm ? S.perm[sr] : sr] : 0u;
+    const unsigned full = __ballot_sync(0xffffffffu, mylen == len);
+    const int ref = full ? __ffs(full) - 1 : 0;
+    bool ok = full != 0 && len > 0 && len <= uint32_t(kSellPatternSlots);
+    uint32_t k = 0;
+    for (uint32_t j = 0; j < len && ok; ++j) {
+      const int64_t mine = int64_t(S.col[e0 + j * 32u + ref]) - ref + lane;
+      if (k < mylen && int64_t(S.col[e0 + k * 32u + lane]) == mine) ++k;
+      ok = __all_sync(0xffffffffu, mine >= 0 && mine < int64_t(S.cols));
+    }
+    ok = __all_sync(0xffffffffu, ok && k == mylen);
+    if (lane == 0) S.md[c] = ok ? len | uint32_t(ref + 1) << 23 : 0u;
+  }
+}
+
+// a candidate chunk against pattern p: the offsets of its reference row (lane j holds slot j's)
+__device__ __forceinline__ bool sell_follows(const SellSetup& S, const int32_t* pat, uint32_t plen, int32_t off,
+                                             uint32_t len, uint32_t lane) {
+  return __all_sync(0xffffffffu, plen == len && (lane >= len || pat[lane] == off));
+}
+__device__ __forceinline__ int32_t sell_offset(const SellSetup& S, uint32_t c, uint32_t md, uint32_t lane) {
+  const uint32_t len = md & 0x7fffffu, ref = ((md >> 23) & 63u) - 1u;
+  return lane < len ? int32_t(S.col[S.cs[c] + lane * 32u + ref] - (c * 32u + ref)) : 0;
+}
+
+// pass 1 (one CTA per matrix): the patterns of the candidates in the kSellScan chunks from the
+// middle of the matrix on, each the first that follows none of the earlier ones
+constexpr uint32_t kSellScan = 512;
+__global__ void __launch_bounds__(1024) k_sell_patterns(const SellSetup* all) {
+  const SellSetup S = all[blockIdx.x];
+  __shared__ uint32_t first;
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t c0 = S.nchunks > kSellScan ? (S.nchunks - kSellScan) / 2 : 0u;
+  const uint32_t c1 = S.nchunks - c0 < kSellScan ? S.nchunks : c0 + kSellScan;
+  for (int p = 0; p < kSellPatterns; ++p) {
+    if (threadIdx.x == 0) first = 0xffffffffu;
+    __syncthreads();
+    for (uint32_t c = c0 + w; c < c1; c += 32) {
+      const uint32_t md = S.md[c];
+      bool fresh = md != 0u;
+      const int32_t off = fresh ? sell_offset(S, c, md, lane) : 0;
+      for (int q = 0; q < p && fresh; ++q)
+        fresh = !sell_follows(S, S.pat + q * kSellPatternSlots, S.plen[q], off, md & 0x7fffffu, lane);
+      if (fresh) {
+        if (lane == 0) atomicMin(&first, c);
+        break;
+      }
+    }
+    __syncthreads();
+    const uint32_t c = first;
+    if (c == 0xffffffffu) break;
+    if (w == 0) {
+      const uint32_t md = S.md[c];
+      S.pat[p * kSellPatternSlots + lane] = sell_offset(S, c, md, lane);
+      if (lane == 0) S.plen[p] = md & 0x7fffffu;
+    }
+    __syncthreads();
+  }
+}
+
+// pass 2: the final form of every chunk; the entries of the chunks that follow a pattern move
+__global__ void __launch_bounds__(256) k_sell_forms(SellSetup S) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < S.nchunks; c += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t md = S.md[c], e0 = S.cs[c], len = S.cl[c], sr = c * 32u + lane;
+    uint32_t form = 0;
+    if (md) {
+      const int32_t off = sell_offset(S, c, md, lane);
+      for (int p = 0; p < kSellPatterns && !form; ++p)
+        if (sell_follows(S, S.pat + p * kSellPatternSlots, S.plen[p], off, len, lane)) form = p + 1;
+    }
+    __syncwarp();
+    if (lane == 0) S.md[c] = len | (form << 28);
+    if (!form) continue;
+    const uint32_t mylen = sr < S.rows ? S.rl[S.perm ? S.perm[sr] : sr] : 0u;
+    uint32_t* cp = S.col + e0 + lane;
+    double* vp = S.val + e0 + lane;
+    uint32_t k = mylen;  // from the last slot down: an entry only moves to a slot at or behind its own
+    for (uint32_t j = len; j-- > 0;) {
+      const uint32_t at = sr + uint32_t(S.pat[(form - 1) * kSellPatternSlots + j]);
+      const bool here = k > 0 && cp[(k - 1u) * 32u] == at;
+      const double v = here ? vp[(k - 1u) * 32u] : 0.0;
+      if (here) --k;
+      cp[j * 32u] = here ? at : 0xffffffffu;
+      vp[j * 32u] = v;
+    }
+  }
+}
+
+// the forms of the levels whose operator runs on the SELL matrix, all levels at once
+static int ensure_sell_forms(fb_mg* m) {
+  std::vector<DevSell*> todo;
+  uint64_t chunks = 0;
+  for (auto& L : m->L) {
+    // (levels of the dense small end's size: no gain for the setup's launches)
+    if (use_matfree(m, L) || use_stencil(m, L) || L.A.md || !L.A.v64 || L.n <= kDenseRows) continue;
+    todo.push_back(&L.A);
+    chunks += L.A.nchunks;
+  }
+  if (todo.empty()) return FB_OK;
+  constexpr size_t kPat = kSellPatterns * kSellPatternSlots, kTab = kPat + kSellPatterns;
+  const size_t nt = todo.size();
+  uint32_t *md = nullptr, *tab = nullptr;
+  SellSetup* dset = nullptr;
+  FB_TRY(dalloc(m, &md, chunks));
+  FB_TRY(dalloc(m, &tab, kTab * nt));
+  FB_CUDA(cudaMemsetAsync(tab, 0, sizeof(uint32_t) * kTab * nt, m->stream));
+  std::vector<SellSetup> set(nt);
+  uint64_t at = 0;
+  for (size_t i = 0; i < nt; ++i) {
+    DevSell& S = *todo[i];
+    uint32_t* t = tab + kTab * i;
+    set[i] = {S.rows, S.cols, S.nchunks, S.cs, S.cl, S.rl, S.perm, S.col, S.v64, md + at, reinterpret_cast<int32_t*>(t), t + kPat};
+    at += S.nchunks;
+    k_sell_candidates<<<ew_grid(uint64_t(S.nchunks) * 32), 256, 0, m->stream>>>(set[i]);
+    FB_CHECK_LAUNCH();
+  }
+  FB_TRY(dupload(m, &dset, set.data(), nt));
+  k_sell_patterns<<<unsigned(nt), 1024, 0, m->stream>>>(dset);
+  FB_CHECK_LAUNCH();
+  for (size_t i = 0; i < nt; ++i) {
+    k_sell_forms<<<ew_grid(uint64_t(todo[i]->nchunks) * 32), 256, 0, m->stream>>>(set[i]);
+    FB_CHECK_LAUNCH();
+  }
+  std::vector<uint32_t> h(kTab * nt);
+  FB_CUDA(cudaMemcpyAsync(h.data(), tab, sizeof(uint32_t) * h.size(), cudaMemcpyDeviceToHost, m->stream));
+  FB_CUDA(cudaStreamSynchronize(m->stream));
+  for (size_t i = 0; i < nt; ++i) {
+    std::memcpy(todo[i]->pat, h.data() + kTab * i, sizeof(todo[i]->pat));
+    todo[i]->md = set[i].md;
+  }
+  return FB_OK;
+}
+
 static int ensure_vectors(fb_mg* m, int prec) {
   if (m->prec_built == prec) return FB_OK;
   const int nl = (int)m->L.size();
   const bool low = prec != FB_PREC_F64;
+  FB_TRY(ensure_sell_forms(m));  // before the value copies, which follow its order of the entries
   for (int l = 0; l < nl; ++l) {
     Level& L = m->L[l];
     if (!low && !L.x64) {

@@ -3,6 +3,7 @@
 #include <cstddef>
 #include "fb_sell.cuh"
 
+#include <cstring>
 #include <vector>
 
 namespace fb {
@@ -35,15 +36,18 @@ struct DevSell {
   uint64_t nnz = 0;       // true nonzeros
   uint32_t *cs = nullptr, *cl = nullptr, *col = nullptr, *perm = nullptr;
   uint32_t* rl = nullptr;   // row lengths (setup / export only)
+  uint32_t* md = nullptr;   // chunk forms (SellView), built when a kernel first needs them (ensure_sell_forms)
+  int32_t pat[kSellPatterns][kSellPatternSlots] = {};
   double* v64 = nullptr;
   float* v32 = nullptr;
   __half* v16 = nullptr;
   float scale16 = 1.0f;
   SellView view(int prec) const {
     SellView v;
-    v.nchunks = nchunks; v.rows = rows; v.cs = cs; v.cl = cl; v.col = col; v.perm = perm;
+    v.nchunks = nchunks; v.rows = rows; v.cs = cs; v.cl = cl; v.md = md ? md : cl; v.col = col; v.perm = perm;
     v.val = prec == FB_PREC_F64 ? (const void*)v64 : (prec == FB_PREC_F32 ? (const void*)v32 : (const void*)v16);
     v.scale = prec == FB_PREC_F16 ? scale16 : 1.0f;
+    std::memcpy(v.pat, pat, sizeof(pat));
     return v;
   }
 };

@@ -6,6 +6,10 @@
 // The kernels are grid-stride over chunks with a grid sized to the resident capacity of the
 // 148 SMs, and finish with an "epilogue" functor that fuses what follows the product in the
 // reference's operator sequence (defect, Jacobi update, filter, dot products).
+//
+// A chunk whose 32 rows have their columns at the same offsets from the row (lattice matrices)
+// refers to one of a few offset patterns, which are kernel parameters, and reads no column
+// indices; the others read a 32-bit column per entry (k_sell_forms finds the patterns).
 #pragma once
 #include "fb_common.cuh"
 
@@ -44,15 +48,21 @@ __device__ __forceinline__ float2 ld_stream_pair(const __half* p) {
   return __half22float2(*reinterpret_cast<const __half2*>(&u));
 }
 
+constexpr int kSellPatterns = 4;       // offset patterns per matrix
+constexpr int kSellPatternSlots = 32;  // longest chunk that may follow a pattern
+constexpr uint32_t kSellLen = 0x0fffffffu;
+
 struct SellView {
   uint32_t nchunks;
   uint32_t rows;
   const uint32_t* cs;    // nchunks+1 chunk starts (entries)
   const uint32_t* cl;    // nchunks chunk lengths (slots)
+  const uint32_t* md;    // per chunk: length | (pattern + 1) << 28, 0 << 28 = columns from col
   const uint32_t* col;   // column per entry
   const void* val;       // values (double / float / __half; FP16: slot pairs interleaved, see k_sell)
   const uint32_t* perm;  // slot row -> matrix row (nullptr = identity)
   float scale;           // FP16 storage: a_ij = scale * h_ij (1 otherwise)
+  int32_t pat[kSellPatterns][kSellPatternSlots];  // column - slot row, per pattern and slot
 };
 
 __device__ __forceinline__ bool masked(const uint32_t* mask, uint32_t row) {
@@ -194,8 +204,8 @@ struct EpiProlong {
 // arithmetic is the epilogue's own. Epilogues without a specialisation load nothing ahead, and
 // neither do the kernels that measured slower with it: the FP64 and FP32 SELL steps (926 -> 991
 // and 652 -> 659 us per Jacobi step at 257^3) and the FP64 stencil Jacobi step (647 -> 656 us,
-// EpiPreIf<false, ...>). Measured faster: the FP32 packed stencil step 365 -> 349 us, the FP64
-// stencil PCG-q 656 -> 639 us, the FP16 SELL step 527 -> 520 us.
+// EpiPreIf<false, ...>). Measured faster: the FP32 packed stencil step 365 -> 349 us and the FP64
+// stencil PCG-q 656 -> 639 us.
 template<typename Epi>
 struct EpiPreNone {
   struct type {};
@@ -272,76 +282,88 @@ struct EpiFiltered {
 };
 
 // ------------------------------------------------------------------ SELL kernel
-// AT = accumulation type (double for FP64 values, float otherwise)
-template<typename VT, typename XT, typename AT, typename Epi, int UNROLL>
-__global__ void __launch_bounds__(256) k_sell(SellView A, const XT* __restrict__ x, Epi epi,
+// adds the products of U slots from slot j on: the loads of all of them, then the sum in slot order
+template<int U, bool PAT, typename VT, typename XT, typename AT>
+__device__ __forceinline__ void sell_group(AT& sum, const uint32_t* __restrict__ col, const int32_t* pat,
+                                           const VT* __restrict__ val, const VT* __restrict__ vpair,
+                                           const XT* __restrict__ x, uint32_t srow, uint32_t j) {
+  uint32_t cc[U];
+  AT vv[U];
+  XT xx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) cc[u] = PAT ? srow + uint32_t(pat[j + u]) : ld_stream(col + (j + u) * 32u);
+  if constexpr (sizeof(VT) == 2 && U > 1) {
+    static_assert(U % 2 == 0, "slot pairs");
+#pragma unroll
+    for (int u = 0; u < U; u += 2) {
+      const float2 v = ld_stream_pair(vpair + (j + u) * 32u);
+      vv[u] = AT(v.x);
+      vv[u + 1] = AT(v.y);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) vv[u] = AT(ld_stream(val + (j + u) * 32u));
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) xx[u] = __ldg(x + cc[u]);
+#pragma unroll
+  for (int u = 0; u < U; ++u) sum += vv[u] * AT(xx[u]);
+}
+
+// sum of a lane's products over its chunk's slots, in slot order; cs = the chunk's first entry,
+// srow = the lane's slot row, pat = the chunk's offsets (PAT)
+template<typename VT, typename XT, typename AT, int U, bool PAT>
+__device__ __forceinline__ AT sell_sum(const SellView& A, const int32_t* pat, const XT* __restrict__ x, uint32_t cs,
+                                       uint32_t len, uint32_t srow, uint32_t lane) {
+  const VT* __restrict__ v = static_cast<const VT*>(A.val) + cs + lane;
+  // FP16: slots 2p and 2p+1 of a chunk are stored interleaved (entry cs + 64p + 2 lane + (j & 1)),
+  // so one 4-byte load per lane brings both values; an odd last slot keeps the plain layout
+  const VT* __restrict__ vp = v + lane;
+  const uint32_t* __restrict__ col = A.col + cs + lane;
+  AT sum = AT(0);
+  uint32_t j = 0;
+  if constexpr (sizeof(VT) == 2) {
+    for (; j + U <= len; j += U) sell_group<U, PAT>(sum, col, pat, v, vp, x, srow, j);
+    for (; j + 2 <= len; j += 2) sell_group<2, PAT>(sum, col, pat, v, vp, x, srow, j);
+  } else {
+    for (; j + U <= len; j += U) sell_group<U, PAT>(sum, col, pat, v, vp, x, srow, j);
+    for (; j + 3 <= len; j += 3) sell_group<3, PAT>(sum, col, pat, v, vp, x, srow, j);
+  }
+  for (; j < len; ++j) sell_group<1, PAT>(sum, col, pat, v, vp, x, srow, j);
+  return sum;
+}
+
+// AT = accumulation type (double for FP64 values, float otherwise). A chunk's start and form are
+// loaded one chunk ahead. Slots in flight per lane (U) and the register budget (CTAs per SM) as
+// measured at 257^3, Jacobi step / defect / PCG-q: FP64 8 slots (9 for PCG-q) in at most 64
+// registers 649 / 617 / 619 us (32 registers 648 / 631 / 619, no bound 730 / 668 / 712); FP32 8 slots
+// in 32 registers 398 / 382 us (no bound 595 / 519); FP16 12 slots without a bound 359 / 314 us (8
+// slots 463 / 404, 14 slots in 32 registers 407 / 356). With a 32-bit column read per entry the same
+// steps took 909 / 889 / 874, 644 / 640 and 516 / 642 us. FP64 streams 4.2 GB per Jacobi step, 6.5
+// TB/s; FP32 and FP16 are bound by their x loads' issue, not by the bytes.
+template<typename VT> constexpr int sell_ctas() { return sizeof(VT) == 8 ? 4 : (sizeof(VT) == 4 ? 8 : 1); }
+template<typename VT, typename XT, typename AT, typename Epi>
+__global__ void __launch_bounds__(256, sell_ctas<VT>()) k_sell(const __grid_constant__ SellView A, const XT* __restrict__ x, Epi epi,
                                               double* ws, unsigned* counter, double* red_out) {
   __shared__ double sh[8];
-  const int lane = threadIdx.x & 31;
-  const uint32_t wpb = blockDim.x >> 5;
-  const VT* __restrict__ val = static_cast<const VT*>(A.val);
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t step = gridDim.x * (blockDim.x >> 5);
+  constexpr int U = sizeof(VT) == 2 ? 12 : (std::is_same<Epi, EpiPcgQ<AT, XT>>::value ? 9 : 8);
   double acc = 0.0;
-  for (uint32_t c = blockIdx.x * wpb + (threadIdx.x >> 5); c < A.nchunks; c += gridDim.x * wpb) {
-    const uint32_t beg = __ldg(A.cs + c) + lane;
-    const uint32_t len = __ldg(A.cl + c);
-    AT sum = AT(0);
-    uint32_t j = 0;
-    if constexpr (sizeof(VT) == 2) {
-      // FP16: slots 2p and 2p+1 of a chunk are stored interleaved (entry cs + 64p + 2 lane + (j & 1)),
-      // so one 4-byte load per lane brings both values; an odd last slot keeps the plain layout.
-      // The products are summed in slot order, as in the plain form. The row and its epilogue
-      // operands are loaded ahead of the products (EpiPre).
-      const uint32_t srow = c * 32u + lane;
-      const bool has = srow < A.rows;
-      const uint32_t row = has ? (A.perm ? __ldg(A.perm + srow) : srow) : 0u;
-      const typename EpiPre<Epi>::type pre = has ? EpiPre<Epi>::load(epi, row) : typename EpiPre<Epi>::type{};
-      const VT* vpair = val + (beg - lane) + 2u * lane;
-      for (; j + 2 <= len; j += 2) {
-        const uint32_t c0 = ld_stream(A.col + beg + j * 32u), c1 = ld_stream(A.col + beg + (j + 1) * 32u);
-        const float2 v = ld_stream_pair(vpair + j * 32u);
-        sum += AT(v.x) * AT(__ldg(x + c0));
-        sum += AT(v.y) * AT(__ldg(x + c1));
-      }
-      for (; j + UNROLL <= len; j += UNROLL) {
-        uint32_t cc[UNROLL];
-        AT vv[UNROLL];
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-          cc[u] = ld_stream(A.col + beg + (j + u) * 32u);
-          vv[u] = AT(ld_stream(val + beg + (j + u) * 32u));
-        }
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) sum += vv[u] * AT(__ldg(x + cc[u]));
-      }
-      for (; j < len; ++j) {
-        const uint32_t cc = ld_stream(A.col + beg + j * 32u);
-        sum += AT(ld_stream(val + beg + j * 32u)) * AT(__ldg(x + cc));
-      }
-      if (has) {
-        sum *= AT(A.scale);
-        acc += EpiPre<Epi>::apply(epi, row, sum, pre);
-      }
-      continue;
+  uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  uint32_t cs = c < A.nchunks ? __ldg(A.cs + c) : 0u, md = c < A.nchunks ? __ldg(A.md + c) : 0u;
+  while (c < A.nchunks) {
+    const uint32_t cs0 = cs, len = md & kSellLen, form = md >> 28, srow = c * 32u + lane;
+    c += step;
+    if (c < A.nchunks) {
+      cs = __ldg(A.cs + c);
+      md = __ldg(A.md + c);
     }
-    for (; j + UNROLL <= len; j += UNROLL) {
-      uint32_t cc[UNROLL];
-      AT vv[UNROLL];
-#pragma unroll
-      for (int u = 0; u < UNROLL; ++u) {
-        cc[u] = ld_stream(A.col + beg + (j + u) * 32u);
-        vv[u] = AT(ld_stream(val + beg + (j + u) * 32u));
-      }
-#pragma unroll
-      for (int u = 0; u < UNROLL; ++u) sum += vv[u] * AT(__ldg(x + cc[u]));
-    }
-    for (; j < len; ++j) {
-      const uint32_t cc = ld_stream(A.col + beg + j * 32u);
-      sum += AT(ld_stream(val + beg + j * 32u)) * AT(__ldg(x + cc));
-    }
-    const uint32_t srow = c * 32u + lane;
+    AT sum = form ? sell_sum<VT, XT, AT, U, true>(A, A.pat[form - 1], x, cs0, len, srow, lane)
+                  : sell_sum<VT, XT, AT, U, false>(A, nullptr, x, cs0, len, srow, lane);
     if (srow < A.rows) {
-      const uint32_t row = A.perm ? __ldg(A.perm + srow) : srow;
-      acc += epi(row, sum);
+      if (sizeof(VT) == 2) sum *= AT(A.scale);
+      acc += epi(A.perm ? __ldg(A.perm + srow) : srow, sum);
     }
   }
   if (Epi::kReduce) {

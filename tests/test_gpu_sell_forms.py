@@ -1,0 +1,108 @@
+"""SELL products on every chunk form: chunks that follow an offset pattern (lattice rows, with gaps
+next to the boundary), more patterns than are kept, and chunks read with their 32-bit columns (sorted
+slots, unsorted columns, long rows, rows without off-diagonal entries). The product and one smoothing
+step against the same in NumPy, and the stored matrix read back entry by entry."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+import torch
+
+pytestmark = pytest.mark.gpu
+
+EPS = {"f64": 2.0 ** -53, "f32": 2.0 ** -24, "f16": 2.0 ** -11}
+
+
+def lattice(shape, degree=1):
+    """pattern of a Q1/Q2 matrix on a lattice with random values, rows in ascending columns"""
+    per = []
+    for m in shape:
+        i = np.arange(m)
+        far = np.where((degree == 1) | (i % 2 == 1), 1, 2)
+        per.append(sp.csr_matrix((np.abs(i[:, None] - i[None, :]) <= far[:, None]).astype(float)))
+    A = per[0]
+    for p in per[1:]:
+        A = sp.kron(A, p, format="csr")
+    A.sort_indices()
+    return A.indptr.astype(np.int64), A.indices.astype(np.int64)
+
+
+def scattered(n, seed, longest=1, shuffle=False):
+    rng = np.random.default_rng(seed)
+    rp, ci = [0], []
+    for i in range(n):
+        k = int(rng.integers(0, longest + 1))
+        c = np.unique(np.append(rng.integers(0, n, k), i))
+        if shuffle:
+            rng.shuffle(c)
+        ci.extend(c)
+        rp.append(len(ci))
+    return np.array(rp), np.array(ci)
+
+
+def bands(n, widths):
+    """blocks of 64 rows, each with its own bandwidth: one pattern per block"""
+    rp, ci = [0], []
+    for i in range(n):
+        w = widths[(i // 64) % len(widths)]
+        ci.extend(c for c in range(i - w, i + w + 1) if 0 <= c < n)
+        rp.append(len(ci))
+    return np.array(rp), np.array(ci)
+
+
+# (a single level above 4,096 rows has no dense inverse to set up)
+CASES = {
+    "q1_2d_70x67": lambda: lattice((67, 70)),
+    "q1_3d_33": lambda: lattice((13, 33, 33)),
+    "q1_3d_17": lambda: lattice((17, 17, 17)),
+    "q2_2d_65": lambda: lattice((65, 65), 2),
+    "q2_3d_17": lambda: lattice((17, 17, 17), 2),      # 125 entries a row: no pattern that long
+    "bands": lambda: bands(64 * 66 + 17, [1, 2, 3, 4, 5, 15, 20]),  # more patterns than kept, one of 41 slots
+    "diagonal": lambda: scattered(4500, 1, 0),
+    "scattered": lambda: scattered(4501, 2, 9),
+    "unsorted": lambda: scattered(4300, 3, 40, True),
+    "one_row": lambda: scattered(1, 4, 0),
+    "partial_chunk": lambda: lattice((4133,)),
+}
+
+
+@pytest.mark.parametrize("sigma", [1, 256])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_products(name, sigma):
+    from feat3_b200.solver import MultiGrid
+    rp, ci = CASES[name]()
+    n = rp.size - 1
+    rng = np.random.default_rng(7)
+    va = rng.uniform(-1.0, 1.0, ci.size)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    va[ci == rows] = 4.0 + rng.uniform(0.0, 1.0, n)
+    A = sp.csr_matrix((va, ci, rp), shape=(n, n), copy=True)
+    absA = abs(A)
+    x, b = rng.standard_normal(n), rng.standard_normal(n)
+    filt = np.arange(0, n, 37) if n > 1 else np.zeros(0, np.int64)
+    keep = np.ones(n)
+    keep[filt] = 0.0
+    mg = MultiGrid.from_csr([{"A": (rp, ci, va), "filter": filt}], sell_sigma=sigma)
+    # one Richardson step with the identity preconditioner: x + filter(b - A x)
+    mg.configure(outer="richardson", coarse="none", max_iter=1, tol=0.0)
+    u = mg.solve(torch.tensor(b).cuda(), torch.tensor(x).cuda())["u"].cpu().numpy()
+    bound = (np.diff(rp) + 3) * EPS["f64"] * (absA @ abs(x) + abs(b) + abs(x))
+    assert np.all(abs(u - (x + keep * (b - A @ x))) <= bound)
+    # two damped Jacobi steps from zero: s + w/a (b - A s), s = w/a b
+    w = 0.5 / A.diagonal()
+    for prec in ("f64", "f32", "f16"):
+        mg.configure(nu=2, coarse="smoother", precision=prec)
+        z = mg.vcycle(torch.tensor(b).cuda()).cpu().numpy()
+        s = keep * w * b
+        ref = keep * (s + w * (b - A @ s))
+        # per entry: the value's rounding, the vector's and one per addition, each relative to its term
+        e = EPS["f32"] if prec != "f64" else EPS["f64"]
+        lim = ((np.diff(rp) + 8) * e + EPS[prec] * 1.01) * (abs(s) + abs(w) * (abs(b) + absA @ abs(s)))
+        # FP16 values below 2^-14 of the scale (5.0 / 2^14 here) lose relative precision: one spacing
+        lim += (5.1 / 2 ** 14 * 2.0 ** -25 * abs(w) * (sp.csr_matrix((np.ones(ci.size), ci, rp), shape=(n, n)) @ abs(s))
+                if prec == "f16" else 0.0)
+        assert np.all(abs(z - ref) <= lim), prec
+    erp, eci, eva = mg.export_csr(0)
+    np.testing.assert_array_equal(erp, rp)
+    np.testing.assert_array_equal(eci, ci)
+    np.testing.assert_array_equal(eva, va)
+    mg.close()
