@@ -7,6 +7,10 @@
 // forms it column by column in FP64 when the solver is configured; a cycle then applies it as one
 // matrix-vector product (dense_rows) in place of some 2 nu + 3 dependent launches per level, each of
 // which costs its latency (2-4 us) for a few KB of work.
+// Whole solves with / without it: 2D Q1 129^2 FP64 V(4,4) 0.65 / 1.19 ms, 65^3 FP64 handed over as CSR
+// 3.55 / 4.29 ms, 2D Q2 1025^2 on FP16 values 19.2 / 22.3 ms, 257^3 mixed matrix-free 14.13 / 14.40 ms
+// (its coarse cluster then runs one level instead of four); it adds 0.7 ms to the configuration. In the
+// FP32 and FP16 forms these levels' matrices enter in FP64 and only the operator is rounded.
 #pragma once
 #include "fb_sell.cuh"
 
@@ -57,16 +61,19 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseArgs D, T* o
     const uint32_t ch = sr >> 5, e = L.A.cs[ch] + (sr & 31u), len = L.A.cl[ch];
     const double* val = static_cast<const double*>(L.A.val);
     double s = 0.0;
+#pragma unroll 4
     for (uint32_t j = 0; j < len; ++j) {
-      const uint32_t cc = __ldg(L.A.col + e + j * 32u);
-      if (cc != 0xffffffffu) s += __ldg(val + e + j * 32u) * x[size_t(cc) * NC + c];
+      const uint32_t cc = __ldg(L.A.col + e + j * 32u);  // an empty slot's value is 0
+      s += __ldg(val + e + j * 32u) * x[(cc == 0xffffffffu ? 0u : cc) * NC + c];
     }
     return s;
   };
   auto transfer = [&](const CsrView& A, const double* x, uint32_t row, uint32_t c) {
     const double* val = static_cast<const double*>(A.val);
+    const uint32_t end = __ldg(A.rp + row + 1);
     double s = 0.0;
-    for (uint32_t k = __ldg(A.rp + row); k < __ldg(A.rp + row + 1); ++k) s += __ldg(val + k) * x[size_t(__ldg(A.col + k)) * NC + c];
+#pragma unroll 4
+    for (uint32_t k = __ldg(A.rp + row); k < end; ++k) s += __ldg(val + k) * x[__ldg(A.col + k) * NC + c];
     return s;
   };
   // one pass over the level's slot rows: f(row, column, A x)

@@ -1051,15 +1051,14 @@ static int build_dense(fb_mg* m, T** op) {
     if (i + 1 < D.nlv) { D.L[i].P = L.P.view(false); D.L[i].R = L.R.view(false); }
     rows += L.n;
   }
-  // NC unit vectors per CTA: as many of 4, 2, 1 as the level vectors leave room for
+  // NC unit vectors per CTA: 2 where the level vectors leave room for them (at most 3 CTAs per SM)
   const size_t per = size_t(rows) * 3 * sizeof(double), cap = 220 * 1024;
   if (per > cap) return FB_OK;
   const uint32_t n = m->L[ld].n;
   const uint64_t size = uint64_t(n) * dense_ld(n);
   if (!*op && dalloc(m, op, size) != FB_OK) return FB_OK;  // no room: level by level
   FB_CUDA(cudaMemsetAsync(*op, 0, sizeof(T) * size, m->stream));
-  if (4 * per <= cap) FB_TRY((launch_dense_build<T, 4>(m, D, *op, 4 * per)));
-  else if (2 * per <= cap) FB_TRY((launch_dense_build<T, 2>(m, D, *op, 2 * per)));
+  if (2 * per <= cap) FB_TRY((launch_dense_build<T, 2>(m, D, *op, 2 * per)));
   else FB_TRY((launch_dense_build<T, 1>(m, D, *op, per)));
   m->dense_l = ld;
   return FB_OK;
@@ -1664,8 +1663,9 @@ __device__ __forceinline__ int32_t sell_offset(const SellSetup& S, uint32_t c, u
 // pass 1 (one CTA per matrix): the patterns of the candidates in the kSellScan chunks from the
 // middle of the matrix on, each the first that follows none of the earlier ones
 constexpr uint32_t kSellScan = 512;
-__global__ void __launch_bounds__(1024) k_sell_patterns(const SellSetup* all) {
-  const SellSetup S = all[blockIdx.x];
+struct SellSetups { SellSetup s[kMaxLevels]; };
+__global__ void __launch_bounds__(1024) k_sell_patterns(const __grid_constant__ SellSetups all) {
+  const SellSetup& S = all.s[blockIdx.x];
   __shared__ uint32_t first;
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t c0 = S.nchunks > kSellScan ? (S.nchunks - kSellScan) / 2 : 0u;
@@ -1738,12 +1738,12 @@ static int ensure_sell_forms(fb_mg* m) {
   if (todo.empty()) return FB_OK;
   constexpr size_t kPat = kSellPatterns * kSellPatternSlots, kTab = kPat + kSellPatterns;
   const size_t nt = todo.size();
-  uint32_t *md = nullptr, *tab = nullptr;
-  SellSetup* dset = nullptr;
-  FB_TRY(dalloc(m, &md, chunks));
-  FB_TRY(dalloc(m, &tab, kTab * nt));
+  uint32_t* tab = nullptr;
+  FB_TRY(dalloc(m, &tab, kTab * nt + chunks));
+  uint32_t* md = tab + kTab * nt;
   FB_CUDA(cudaMemsetAsync(tab, 0, sizeof(uint32_t) * kTab * nt, m->stream));
-  std::vector<SellSetup> set(nt);
+  SellSetups setups{};
+  SellSetup* set = setups.s;
   uint64_t at = 0;
   for (size_t i = 0; i < nt; ++i) {
     DevSell& S = *todo[i];
@@ -1753,8 +1753,7 @@ static int ensure_sell_forms(fb_mg* m) {
     k_sell_candidates<<<ew_grid(uint64_t(S.nchunks) * 32), 256, 0, m->stream>>>(set[i]);
     FB_CHECK_LAUNCH();
   }
-  FB_TRY(dupload(m, &dset, set.data(), nt));
-  k_sell_patterns<<<unsigned(nt), 1024, 0, m->stream>>>(dset);
+  k_sell_patterns<<<unsigned(nt), 1024, 0, m->stream>>>(setups);
   FB_CHECK_LAUNCH();
   for (size_t i = 0; i < nt; ++i) {
     k_sell_forms<<<ew_grid(uint64_t(todo[i]->nchunks) * 32), 256, 0, m->stream>>>(set[i]);
