@@ -380,6 +380,33 @@ struct CsrView {
   const void* val;
 };
 
+// Part of a CSR row's product by lane `sub` of the G that share the row: entries beg + sub,
+// beg + sub + G, ... in this order. The loads of four of them are issued together (past the row's
+// end: its last entry again, not summed), so a lane waits for memory twice per four entries.
+template<int G, typename VT, typename XT, typename AT, typename IT>
+__device__ __forceinline__ AT csr_row(const VT* __restrict__ val, const IT* __restrict__ col, const XT* __restrict__ x,
+                                      IT beg, IT end, int sub) {
+  constexpr int U = 4;
+  AT sum(0);
+  for (IT k = beg + IT(sub); k < end; k += IT(U * G)) {
+    IT cc[U];
+    AT vv[U];
+    XT xx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const IT at = k + IT(u * G) < end ? k + IT(u * G) : end - IT(1);
+      cc[u] = __ldg(col + at);
+      vv[u] = AT(ValLoad<VT>::ld(val + at));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) xx[u] = __ldg(x + cc[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + IT(u * G) < end) sum += vv[u] * AT(xx[u]);
+  }
+  return sum;
+}
+
 template<typename VT, typename XT, typename AT, typename Epi, int G>
 __global__ void __launch_bounds__(256) k_csr_epi(CsrView A, const XT* __restrict__ x, Epi epi,
                                                  double* ws, unsigned* counter, double* red_out) {
@@ -393,11 +420,7 @@ __global__ void __launch_bounds__(256) k_csr_epi(CsrView A, const XT* __restrict
   for (uint32_t rb = blockIdx.x * gpb; rb < A.rows; rb += stride) {
     const uint32_t row = rb + threadIdx.x / G;
     AT sum = AT(0);
-    if (row < A.rows) {
-      const uint32_t end = __ldg(A.rp + row + 1);
-      for (uint32_t k = __ldg(A.rp + row) + sub; k < end; k += G)
-        sum += AT(ValLoad<VT>::ld(val + k)) * AT(__ldg(x + __ldg(A.col + k)));
-    }
+    if (row < A.rows) sum = csr_row<G, VT, XT, AT>(val, A.col, x, __ldg(A.rp + row), __ldg(A.rp + row + 1), sub);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, G);
     if (sub == 0 && row < A.rows) acc += epi(row, sum);

@@ -1,10 +1,10 @@
 // Sparse matrix-vector products of the operator layer:
-//   * CSR  r = b*y + a*A*x   (sub-warp per row, width picked from the mean row length)
+//   * CSR  r = b*y + a*A*x   (1 to 32 threads per row, picked from the mean row length)
 //   * CSR  r = b*y + a*A^T*x (scatter with FP64/FP32 atomics)
 //   * FEAT SELL-C ("ELL") r = b*y + a*A*x (thread per row, chunk-major coalesced streams)
 // Each takes 32-bit (IT = uint32_t) or 64-bit (IT = uint64_t, FEAT's default Index) index
 // arrays as they are; the 64-bit forms read the caller's arrays directly, no narrowing copy.
-#include "fb_common.cuh"
+#include "fb_sell.cuh"
 
 namespace fb {
 
@@ -16,16 +16,13 @@ __global__ void __launch_bounds__(256) k_csr(T* r, T a, const T* __restrict__ x,
   const uint64_t row = gid / G;
   const int sub = threadIdx.x % G;
   if (row >= rows) return;  // whole sub-group exits together (G divides 32)
-  const IT beg = rp[row], end = rp[row + 1];
-  T sum(0);
-  for (IT k = beg + sub; k < end; k += G) sum += val[k] * x[col[k]];
+  T prev(0);
+  if (use_y && sub == 0) prev = y[row];
+  T sum = csr_row<G, T, T, T>(val, col, x, __ldg(rp + row), __ldg(rp + row + 1), sub);
   const unsigned mask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o, G);
-  if (sub == 0) {
-    const T prev = use_y ? y[row] : T(0);
-    r[row] = use_y ? (sum * a) + (b * prev) : sum * a;
-  }
+  if (sub == 0) r[row] = use_y ? (sum * a) + (b * prev) : sum * a;
 }
 
 template<typename T>
@@ -84,12 +81,25 @@ int csr_apply(T* r, T a, const T* x, T b, const T* y, const T* val, const IT* co
     }
     return FB_OK;
   }
+  // Threads per row from the mean row length: about four to seven entries per thread, which loads
+  // four at a time (csr_row). Entries of 12 bytes and more (index and value) take twice the threads on
+  // long rows. Measured (us, threads per row):
+  //   27 entries, 1.03M rows: FP64 u64 82 (8), 90 (4), 127 (16); FP64 u32 72 (8), 75 (4); FP32 u32 58 (4),
+  //   75 (8), 135 (16); 16 entries, 1.0M rows, FP64 u64: 60 (4), 68 (8), 82 (2); 9 entries, 1.44M rows,
+  //   FP64 u32: 45 (2), 49 (4), 84 (8); 3.4 entries, 2.1M rows, FP32 u32: 17 (1), 33 (2), 51 (4)
+  // One entry at a time with 8 threads per row (2 for the last) took 117, 103, 109, 94, 98 and 39 us.
   const double avg = rows ? double(nnz) / double(rows) : 0.0;
-  if (avg <= 4.0)       k_csr<T, 2, IT><<<grid_for(rows * 2, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
-  else if (avg <= 8.0)  k_csr<T, 4, IT><<<grid_for(rows * 4, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
-  else if (avg <= 32.0) k_csr<T, 8, IT><<<grid_for(rows * 8, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
-  else if (avg <= 64.0) k_csr<T, 16, IT><<<grid_for(rows * 16, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
-  else                  k_csr<T, 32, IT><<<grid_for(rows * 32, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
+  constexpr bool wide = sizeof(T) + sizeof(IT) >= 12;
+  auto launch = [&](auto g) {
+    constexpr int G = decltype(g)::value;
+    k_csr<T, G, IT><<<grid_for(rows * G, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
+  };
+  if (avg <= 4.0) launch(std::integral_constant<int, 1>());
+  else if (avg <= 12.0) launch(std::integral_constant<int, 2>());
+  else if (avg <= 20.0) launch(std::integral_constant<int, 4>());
+  else if (avg <= 32.0) launch(std::integral_constant<int, wide ? 8 : 4>());
+  else if (avg <= 64.0) launch(std::integral_constant<int, wide ? 16 : 8>());
+  else launch(std::integral_constant<int, 32>());
   FB_CHECK_LAUNCH();
   return FB_OK;
 }

@@ -1,0 +1,41 @@
+"""CSR products over every width the kernel picks (1 to 32 threads per row, four entries of a thread
+loaded at a time): rows shorter and longer than a group's step, empty rows, rows of very different
+length, both index widths, with and without y, against SciPy in 64 bits."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = {
+    "empty_and_1": lambda rng, n: rng.integers(0, 2, n),
+    "1_to_8": lambda rng, n: rng.integers(1, 9, n),
+    "9": lambda rng, n: np.full(n, 9),
+    "13_to_20": lambda rng, n: rng.integers(13, 21, n),
+    "27": lambda rng, n: np.full(n, 27),
+    "33_to_60": lambda rng, n: rng.integers(33, 61, n),
+    "125": lambda rng, n: np.full(n, 125),
+    "one_long": lambda rng, n: np.where(np.arange(n) == n // 2, 1500, rng.integers(0, 4, n)),
+}
+
+
+@pytest.mark.parametrize("index", ["u32", "u64"])
+@pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
+@pytest.mark.parametrize("name", sorted(LENGTHS))
+def test_rows(name, dtype, eps, index):
+    from feat3_b200.lafem import DenseVector, SparseMatrixCSR
+    rng = np.random.default_rng(3)
+    n, m = 777, 2000
+    rl = LENGTHS[name](rng, n)
+    rp = np.concatenate([[0], np.cumsum(rl)])
+    ci = np.concatenate([np.sort(rng.choice(m, k, replace=False)) for k in rl] + [np.zeros(0, np.int64)]).astype(np.int64)
+    cast = (lambda a: a.astype(np.float32).astype(np.float64)) if dtype == torch.float32 else (lambda a: a)
+    va, x, y = cast(rng.standard_normal(ci.size)), cast(rng.standard_normal(m)), cast(rng.standard_normal(n))
+    S = sp.csr_matrix((va, ci, rp), shape=(n, m), copy=True)
+    A = SparseMatrixCSR(rp, ci, va, columns=m, dtype=dtype, index=index)
+    X, Y, R = (DenseVector(torch.tensor(v, dtype=dtype).cuda()) for v in (x, y, np.full(n, np.nan)))
+    terms = sp.csr_matrix((abs(va), ci, rp), shape=(n, m)) @ abs(x)
+    bound = (rl + 3) * eps * (terms + abs(y))  # one rounding per entry, three for a, b and the sum
+    assert np.all(abs(A.apply(R, X).numpy() - S @ x) <= bound)
+    assert np.all(abs(A.apply(R, X, Y, -1.0).numpy() - (y - S @ x)) <= bound)
