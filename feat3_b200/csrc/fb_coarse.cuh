@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_coarse_cycle(CoarseArgs<T> A) {
     if (A.coarse == FB_COARSE_DIRECT) {
       for (uint32_t i = threadIdx.x; i < A.ldc; i += THREADS) sb[i] = i < L.n ? ldc(b + i) : T(0);
       __syncthreads();
-      dense_rows(A.cinv, A.ldc, sb, L.n, gt >> 5, gs >> 5, gt & 31, [&](uint32_t row, double s) { L.x[row] = T(s); });
+      dense_rows<4>(A.cinv, A.ldc, sb, L.n, gt >> 5, gs >> 5, gt & 31, [&](uint32_t row, double s) { L.x[row] = T(s); });
       cl.sync();
       sol[l] = L.x;
     } else if (A.coarse == FB_COARSE_SMOOTHER) {

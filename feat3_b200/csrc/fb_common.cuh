@@ -26,9 +26,10 @@ void debug_report(cudaError_t e, const char* what, const char* file, int line);
 // Programmatic dependent launch: kernels of the solve path may be scheduled while their
 // predecessor in the stream finishes. Every kernel launched that way starts with pdl_wait()
 // (returns once the predecessor has completed and its writes are visible; a no-op for a
-// normal launch), and signals pdl_trigger() when the rest of its work no longer delays the
-// launch of its successor. Off by default (no gain measured on the graph-replayed solve);
-// FB_PDL=1 in the environment turns the attribute on.
+// normal launch), before which it reads nothing that a launch writes, and signals pdl_trigger()
+// when its successor may be scheduled: at once where grids are small enough to sit beside each
+// other, behind the main loop in the staged kernels. The driver sets the attribute on small grids
+// (launch_pdl in fb_mg.cu); FB_PDL=1 in the environment sets it on every launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 bool pdl_enabled();

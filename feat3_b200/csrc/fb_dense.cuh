@@ -156,50 +156,51 @@ __global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseArgs D, T* o
     if (col0 + i % NC < D.L[0].n) op[size_t(i / NC) * ld + col0 + i % NC] = T(sol[0][i]);
 }
 
-// Dense product rows row0, row0 + stride, ... < n by a warp, kDenseR rows at a time (their loads
-// in flight together); b in shared memory, zeros behind entry n up to ld. 16-byte loads of the
+// Dense product rows row0, row0 + stride, ... < n by a warp, R rows at a time (their loads in flight
+// together); b in shared memory, zeros behind entry n up to ld. 16-byte loads of the
 // operator's rows, whose ld is a multiple of 4 with zeros behind column n; summed in FP64, in the same
 // order for every caller. out(row, sum) runs in lane 0.
-constexpr int kDenseR = 4;
-template<typename T, typename Out>
+template<int R, typename T, typename Out>
 __device__ __forceinline__ void dense_rows(const T* __restrict__ op, uint32_t ld, const T* b, uint32_t n, uint32_t row0,
                                            uint32_t stride, uint32_t lane, Out&& out) {
   constexpr uint32_t NV = 16 / sizeof(T);
-  for (uint32_t r = row0; r < n; r += kDenseR * stride) {
-    double s[kDenseR] = {};
-#pragma unroll 2
+  for (uint32_t r = row0; r < n; r += R * stride) {
+    double s[R] = {};
+#pragma unroll (R > 1 ? 2 : 8)
     for (uint32_t j = lane * NV; j < ld; j += 32 * NV) {
-      T a[kDenseR][NV], bv[NV];
+      T a[R][NV], bv[NV];
 #pragma unroll
-      for (int q = 0; q < kDenseR; ++q)
+      for (int q = 0; q < R; ++q)
         if (r + q * stride < n)
           *reinterpret_cast<float4*>(a[q]) = __ldg(reinterpret_cast<const float4*>(op + size_t(r + q * stride) * ld + j));
       *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(b + j);
 #pragma unroll
-      for (int q = 0; q < kDenseR; ++q)
+      for (int q = 0; q < R; ++q)
         if (r + q * stride < n)
 #pragma unroll
           for (uint32_t v = 0; v < NV; ++v) s[q] += double(a[q][v]) * double(bv[v]);
     }
 #pragma unroll
-    for (int q = 0; q < kDenseR; ++q) {
+    for (int q = 0; q < R; ++q) {
       const double t = warp_sum(s[q]);
       if (lane == 0 && r + q * stride < n) out(r + q * stride, t);
     }
   }
 }
 
-// dense product x = op b (the coarse direct solve, or the small end of the cycle): kDenseR rows per
-// warp; b staged in shared memory (at most 32 KB: a direct solve of 4096 rows in FP64)
+// dense product x = op b (the coarse direct solve, or the small end of the cycle): one row per warp; b
+// staged in shared memory (at most 32 KB: a direct solve of 4096 rows in FP64)
 template<typename T>
 __global__ void __launch_bounds__(128) k_dense_solve(T* x, const T* __restrict__ op, uint32_t ld, const T* __restrict__ b,
                                                      uint32_t n) {
   extern __shared__ __align__(16) unsigned char dense_sm[];
   T* sb = reinterpret_cast<T*>(dense_sm);
+  pdl_wait();
+  pdl_trigger();
   for (uint32_t i = threadIdx.x; i < ld; i += 128) sb[i] = i < n ? b[i] : T(0);
   __syncthreads();
   const uint32_t warp = (blockIdx.x * 128 + threadIdx.x) >> 5, nw = gridDim.x * 4;
-  dense_rows(op, ld, sb, n, warp, nw, threadIdx.x & 31, [&](uint32_t row, double s) { x[row] = T(s); });
+  dense_rows<1>(op, ld, sb, n, warp, nw, threadIdx.x & 31, [&](uint32_t row, double s) { x[row] = T(s); });
 }
 
 }  // namespace fb

@@ -50,7 +50,13 @@ static int occupancy_grid(const void* fn, uint64_t work_warps) {
   return int(g < 1 ? 1 : g);
 }
 
-// launch with the programmatic-dependent-launch attribute (the kernel begins with pdl_wait())
+// Launch with the programmatic-dependent-launch attribute where the grid is small (the kernel
+// begins with pdl_wait()): at most two CTAs per SM, so the grid can sit beside its predecessor's
+// and its launch latency, which such a kernel mostly consists of, overlaps it. Limits of 0 / 150 /
+// 300 / 800 CTAs / none, in us: 2D Q1 129^2 FP64 solve 578 / 528 / 528 / 529 / 527, 65^3 FP64 handed
+// 2832 / 2767 / 2801 / 2750 / 2840, 1025^2 Q2 FP16 13460 / 13120 / 13005 / 13070 / 13055, 129^3 FP32
+// cycle 526 / 504 / 500 / 500 / 475, 257^3 mixed 14350 / 14290 / 14140 / 14150 / 14820.
+constexpr uint64_t kPdlCtas = 300;
 template<typename... KArgs, typename... Args>
 static cudaError_t launch_pdl(cudaStream_t s, void (*fn)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -62,7 +68,8 @@ static cudaError_t launch_pdl(cudaStream_t s, void (*fn)(KArgs...), dim3 grid, d
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  const uint64_t ctas = uint64_t(grid.x) * grid.y * grid.z;
+  cfg.numAttrs = pdl_enabled() || ctas <= kPdlCtas ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, fn, static_cast<KArgs>(args)...);
 }
 
@@ -88,7 +95,7 @@ static int launch_sell(fb_mg* m, const DevSell& A, int prec, const XT* x, const 
   if (debug_enabled())
     debug_check_ptrs("k_sell", {A.cs, A.md, A.col, A.view(prec).val, (const void*)x, (const void*)m->ws,
                                 (const void*)m->counter, (const void*)red_out, (const void*)A.perm});
-  fn<<<grid, 256, 0, m->stream>>>(A.view(prec), x, epi, m->ws, m->counter, red_out);
+  FB_CUDA(launch_pdl(m->stream, fn, dim3(grid), dim3(256), 0, A.view(prec), x, epi, m->ws, m->counter, red_out));
   m->launches++;
   FB_CHECK_LAUNCH();
   return FB_OK;
@@ -103,11 +110,12 @@ static int launch_csr(fb_mg* m, const DevCsr& A, bool f32, const XT* x, const Ep
   auto launch = [&](auto g) {
     constexpr int G = decltype(g)::value;
     auto fn = k_csr_epi<VT, XT, AT, Epi, G>;
-    fn<<<occupancy_grid((const void*)fn, (uint64_t(A.rows) * G + 31) / 32), 256, 0, m->stream>>>(A.view(f32), x, epi, m->ws, m->counter, red_out);
+    const int grid = occupancy_grid((const void*)fn, (uint64_t(A.rows) * G + 31) / 32);
+    return launch_pdl(m->stream, fn, dim3(grid), dim3(256), 0, A.view(f32), x, epi, m->ws, m->counter, red_out);
   };
-  if (avg <= 4.0) launch(std::integral_constant<int, 1>());
-  else if (avg <= 12.0) launch(std::integral_constant<int, 4>());
-  else launch(std::integral_constant<int, 8>());
+  if (avg <= 4.0) FB_CUDA(launch(std::integral_constant<int, 1>()));
+  else if (avg <= 12.0) FB_CUDA(launch(std::integral_constant<int, 4>()));
+  else FB_CUDA(launch(std::integral_constant<int, 8>()));
   m->launches++;
   FB_CHECK_LAUNCH();
   return FB_OK;
@@ -121,7 +129,8 @@ static int launch_stencil_S(fb_mg* m, const DevStencil& St, const void* val, flo
   for (int j = 0; j < S; ++j) v.off[j] = St.off[j];
   constexpr int G = S == 27 ? 9 : S;
   auto fn = k_stencil<VT, XT, AT, Epi, S, G>;
-  fn<<<occupancy_grid((const void*)fn, St.nchunks), 256, 0, m->stream>>>(v, x, epi, m->ws, m->counter, red_out);
+  FB_CUDA(launch_pdl(m->stream, fn, dim3(occupancy_grid((const void*)fn, St.nchunks)), dim3(256), 0, v, x, epi, m->ws,
+                     m->counter, red_out));
   m->launches++;
   FB_CHECK_LAUNCH();
   return FB_OK;
@@ -148,7 +157,8 @@ static int launch_stencil_packed_S(fb_mg* m, const DevStencil& St, const void* v
     if (offsets_are<S, 257>(St, M1)) fn = k_stencil_packed<VT, Epi, S, 257>;
     else if (offsets_are<S, 129>(St, M1)) fn = k_stencil_packed<VT, Epi, S, 129>;
   }
-  fn<<<occupancy_grid((const void*)fn, St.nchunks), 256, 0, m->stream>>>(v, x, epi, m->ws, m->counter, red_out);
+  FB_CUDA(launch_pdl(m->stream, fn, dim3(occupancy_grid((const void*)fn, St.nchunks)), dim3(256), 0, v, x, epi, m->ws,
+                     m->counter, red_out));
   m->launches++;
   FB_CHECK_LAUNCH();
   return FB_OK;
@@ -227,6 +237,8 @@ static int launch_stencil(fb_mg* m, const Level& L, int prec, const XT* x, const
 template<typename T>
 __global__ void k_jacobi0(T* out, const T* __restrict__ b, const T* __restrict__ invd, const uint32_t* mask,
                           const double* skip_src, T omega, uint32_t n) {
+  pdl_wait();
+  pdl_trigger();
   const bool skip = smoother_skip<T>(skip_src);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     out[i] = (skip || masked(mask, i)) ? T(0) : omega * (invd[i] * b[i]);
@@ -941,7 +953,7 @@ static int rest_T(fb_mg* m, int l, const T* xf, const Epi& epi, double* red) {
       }
     }
     const dim3 grid((L.tr.Mc1 + 31) / 32, (L.tr.Mc1 + 7) / 8, L.tr.dim == 3 ? L.tr.Mc1 : 1);
-    k_rest_q1<T, Epi><<<grid, dim3(32, 8), 0, m->stream>>>(L.tr, xf, epi, m->ws, m->counter, red);
+    FB_CUDA(launch_pdl(m->stream, k_rest_q1<T, Epi>, grid, dim3(32, 8), 0, L.tr, xf, epi, m->ws, m->counter, red));
     m->launches++;
     FB_CHECK_LAUNCH();
     return FB_OK;
@@ -970,7 +982,7 @@ static int prol_T(fb_mg* m, int l, const T* xc, const Epi& epi) {
       }
     }
     const dim3 grid((L.tr.Mf1 + 31) / 32, (L.tr.Mf1 + 7) / 8, L.tr.dim == 3 ? L.tr.Mf1 : 1);
-    k_prol_q1<T, Epi><<<grid, dim3(32, 8), 0, m->stream>>>(L.tr, xc, epi);
+    FB_CUDA(launch_pdl(m->stream, k_prol_q1<T, Epi>, grid, dim3(32, 8), 0, L.tr, xc, epi));
     m->launches++;
     FB_CHECK_LAUNCH();
     return FB_OK;
@@ -988,7 +1000,8 @@ static int presmooth(fb_mg* m, int l, const T* b, const double* bnorm, bool need
   T* cur = Prec<T>::x(L);
   T* oth = Prec<T>::y(L);
   if (need_s1) {
-    k_jacobi0<T><<<ew_grid(L.n), 256, 0, m->stream>>>(cur, b, Prec<T>::invd(L), L.mask, bnorm, omega, L.n);
+    FB_CUDA(launch_pdl(m->stream, k_jacobi0<T>, dim3(ew_grid(L.n)), dim3(256), 0, cur, b, (const T*)Prec<T>::invd(L),
+                       (const uint32_t*)L.mask, bnorm, omega, L.n));
     m->launches++;
     FB_CHECK_LAUNCH();
   }
@@ -1014,7 +1027,8 @@ static int launch_dense(fb_mg* m, int l, const T* b) {
   const T* a;
   if constexpr (std::is_same<T, double>::value) a = op ? m->dop64 : m->cinv64; else a = op ? m->dop32 : m->cinv32;
   const uint32_t ld = dense_ld(L.n);
-  k_dense_solve<T><<<grid_for(L.n, 4 * kDenseR), 128, ld * sizeof(T), m->stream>>>(Prec<T>::x(L), a, ld, b, L.n);
+  FB_CUDA(launch_pdl(m->stream, k_dense_solve<T>, dim3(grid_for(L.n, 4)), dim3(128), ld * sizeof(T), Prec<T>::x(L), a, ld, b,
+                     L.n));
   m->launches++;
   FB_CHECK_LAUNCH();
   return FB_OK;
@@ -1156,7 +1170,7 @@ static int launch_coarse(fb_mg* m, int lc, T** sol_lc) {
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = 2;  // (16 CTAs: see launch_pdl)
   if (m->dim == 3) FB_CUDA(cudaLaunchKernelEx(&cfg, k_coarse_cycle<T, 3, coarse_threads<T>()>, A));
   else FB_CUDA(cudaLaunchKernelEx(&cfg, k_coarse_cycle<T, 2, coarse_threads<T>()>, A));
   m->launches++;

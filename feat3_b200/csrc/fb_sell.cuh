@@ -352,6 +352,8 @@ __global__ void __launch_bounds__(256, sell_ctas<VT>()) k_sell(const __grid_cons
   double acc = 0.0;
   uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   uint32_t cs = c < A.nchunks ? __ldg(A.cs + c) : 0u, md = c < A.nchunks ? __ldg(A.md + c) : 0u;
+  pdl_wait();  // (the matrix does not change between launches)
+  pdl_trigger();
   while (c < A.nchunks) {
     const uint32_t cs0 = cs, len = md & kSellLen, form = md >> 28, srow = c * 32u + lane;
     c += step;
@@ -411,6 +413,8 @@ template<typename VT, typename XT, typename AT, typename Epi, int G>
 __global__ void __launch_bounds__(256) k_csr_epi(CsrView A, const XT* __restrict__ x, Epi epi,
                                                  double* ws, unsigned* counter, double* red_out) {
   __shared__ double sh[8];
+  pdl_wait();
+  pdl_trigger();
   const VT* __restrict__ val = static_cast<const VT*>(A.val);
   const int sub = threadIdx.x % G;
   const uint32_t gpb = blockDim.x / G;
@@ -453,6 +457,8 @@ template<typename VT, typename XT, typename AT, typename Epi, int S, int G>
 __global__ void __launch_bounds__(256) k_stencil(StencilView<S> A, const XT* __restrict__ x, Epi epi,
                                                  double* ws, unsigned* counter, double* red_out) {
   __shared__ double sh[8];
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const uint32_t wpb = blockDim.x >> 5;
   const VT* __restrict__ val = static_cast<const VT*>(A.val);
@@ -551,6 +557,8 @@ __global__ void __launch_bounds__(256, 4) k_stencil_packed(StencilView<S> A, con
   constexpr int W = Pack8<VT>::W;
   constexpr int G = (S + W - 1) / W;
   __shared__ double sh[8];
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const uint32_t wpb = blockDim.x >> 5;
   const VT* __restrict__ val = static_cast<const VT*>(A.val);
@@ -630,6 +638,7 @@ __global__ void __launch_bounds__(256) k_mf_q1(MfView<T, DIM> A, const T* __rest
   constexpr int S = DIM == 3 ? 27 : 9;
   constexpr int NE = 1 << DIM;
   pdl_wait();
+  pdl_trigger();
   __shared__ double sh[8];
   const int lane = threadIdx.x & 31;
   const uint32_t wpb = blockDim.x >> 5;
@@ -693,7 +702,6 @@ __global__ void __launch_bounds__(256) k_mf_q1(MfView<T, DIM> A, const T* __rest
     }
     if (row <= last) acc += epi(uint32_t(row), s);
   }
-  pdl_trigger();
   if (Epi::kReduce) {
     const double blk = block_sum<256>(acc, sh);
     reduce_finish<256>(blk, ws, counter, red_out, sh, false);
@@ -730,6 +738,8 @@ struct Q1Transfer {
 // their order are those of the CSR row (plus exact zeros).
 template<typename T, typename Epi>
 __global__ void __launch_bounds__(256) k_prol_q1(Q1Transfer g, const T* __restrict__ xc, Epi epi) {
+  pdl_wait();
+  pdl_trigger();
   const uint32_t X = blockIdx.x * 32 + threadIdx.x, Y = blockIdx.y * 8 + threadIdx.y, Z = blockIdx.z;
   if (X >= g.Mf1 || Y >= g.Mf1) return;
   const uint32_t i = X + g.Mf1 * (Y + g.Mf1 * Z);
@@ -765,6 +775,8 @@ __global__ void __launch_bounds__(256) k_prol_q1(Q1Transfer g, const T* __restri
 template<typename T, typename Epi>
 __global__ void __launch_bounds__(256) k_rest_q1(Q1Transfer g, const T* __restrict__ xf, Epi epi,
                                                  double* ws, unsigned* counter, double* red_out) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ double sh[8];
   const int X = int(blockIdx.x * 32 + threadIdx.x), Y = int(blockIdx.y * 8 + threadIdx.y), Z = int(blockIdx.z);
   double acc = 0.0;
