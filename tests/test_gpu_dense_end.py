@@ -10,7 +10,7 @@ from oracle import pyoracle as po
 pytestmark = pytest.mark.gpu
 
 # dim, degree, level, level_min, nu, coarse
-CASES = [(2, 1, 6, 1, 1, "none"), (2, 1, 7, 2, 3, "smoother"), (2, 1, 6, 4, 2, "direct"), (3, 1, 5, 1, 2, "direct"),
+CASES = [(2, 1, 6, 1, 1, "none"), (2, 1, 7, 1, 2, "direct"), (2, 1, 7, 2, 3, "smoother"), (2, 1, 6, 4, 2, "direct"), (3, 1, 5, 1, 2, "direct"),
          (3, 1, 4, 0, 2, "smoother"), (2, 2, 5, 1, 4, "direct"), (3, 2, 3, 1, 2, "none")]
 
 
