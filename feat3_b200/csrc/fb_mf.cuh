@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(288, MINB) k_mf_q1_tiled(MfView<T, 3> A, MfTil
   pdl_trigger();
   if (Epi::kReduce) {
     const double blk = block_sum<288>(acc, sh);
-    reduce_finish<288>(blk, ws, counter, red_out, sh, false);
+    epi_finish<288>(epi, blk, ws, counter, red_out, sh);
   }
 }
 

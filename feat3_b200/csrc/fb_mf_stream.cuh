@@ -466,7 +466,7 @@ __device__ __forceinline__ void mf_stream_body(const MfView<T, 3>& A, const MfSt
   pdl_trigger();
   if (Epi::kReduce) {
     const double blk = block_sum<NT>(acc, sh);
-    reduce_finish<NT>(blk, ws, counter, red_out, sh, false);
+    epi_finish<NT>(epi, blk, ws, counter, red_out, sh);
   }
 }
 

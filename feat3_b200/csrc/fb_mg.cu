@@ -1204,7 +1204,7 @@ static int vcycle(fb_mg* m, const T* rhs_top, const double* rhs_top_sumsq, T** o
     const bool coarsest_next = (l + 2 == nl);
     T* s1 = nullptr;
     if (nu >= 2 && (!coarsest_next || coarse == FB_COARSE_SMOOTHER)) s1 = Prec<T>::x(C);
-    EpiRestrict<T> er{Prec<T>::rhs(C), s1, Prec<T>::invd(C), C.mask, omega};
+    EpiRestrict<T> er{Prec<T>::rhs(C), s1, Prec<T>::invd(C), C.mask, omega, &m->sc->lvl[2 * l + 1]};
     FB_TRY(rest_T<T>(m, l, Prec<T>::def(L), er, &m->sc->lvl[2 * (l + 1)]));
   }
   // ---- coarse grid (multigrid.hpp:1524-1587)
@@ -1256,7 +1256,7 @@ static int vcycle(fb_mg* m, const T* rhs_top, const double* rhs_top_sumsq, T** o
     double* dn = &m->sc->lvl[2 * l + 1];
     for (int it = 0; it < nu; ++it) {
       if (it == 0) {
-        EpiJacobi<T, true> e{cur, b, Prec<T>::invd(L), oth, nullptr, L.mask, nullptr, omega};
+        EpiJacobi<T, true> e{cur, b, Prec<T>::invd(L), oth, nullptr, L.mask, nullptr, omega, &m->sc->lvl[2 * (l + 1)]};
         FB_TRY(spmv_L<T>(m, L, cur, e, dn));
         if (nu == 1) {
           k_skip_fix<T><<<ew_grid(L.n), 256, 0, m->stream>>>(oth, s0, dn, L.n);
@@ -1313,7 +1313,7 @@ struct Cycle {
     double* dn = &m->sc->lvl[2 * l + 1];
     for (int it = 0; it < nu; ++it) {
       if (it == 0) {
-        EpiJacobi<T, true> e{cur, rhs(l), Prec<T>::invd(L), oth, nullptr, L.mask, nullptr, omega};
+        EpiJacobi<T, true> e{cur, rhs(l), Prec<T>::invd(L), oth, nullptr, L.mask, nullptr, omega, &m->sc->lvl[2 * (l + 1)]};
         FB_TRY(spmv_L<T>(m, L, cur, e, dn));
         if (nu == 1) {
           k_skip_fix<T><<<ew_grid(L.n), 256, 0, m->stream>>>(oth, s0, dn, L.n);
@@ -1341,7 +1341,7 @@ struct Cycle {
       const bool coarsest_next = (i + 2 == nl);
       T* s1 = nullptr;
       if (nu >= 2 && (!coarsest_next || m->cfg.coarse == FB_COARSE_SMOOTHER)) s1 = Prec<T>::x(C);
-      EpiRestrict<T> er{Prec<T>::rhs(C), s1, Prec<T>::invd(C), C.mask, omega};
+      EpiRestrict<T> er{Prec<T>::rhs(C), s1, Prec<T>::invd(C), C.mask, omega, &m->sc->lvl[2 * i + 1]};
       FB_TRY(rest_T<T>(m, i, Prec<T>::def(L), er, &m->sc->lvl[2 * (i + 1)]));
     }
     return FB_OK;
@@ -2097,6 +2097,7 @@ int solve_dev(fb_mg* m, const double* rhs, double* sol, double* hist, fb_solve_i
   cudaStream_t s = m->stream;
   const uint32_t* perm = feat_io ? m->feat_dof : nullptr;
   m->launches = 0;
+  FB_CUDA(cudaMemsetAsync(m->sc->lvl, 0, sizeof(m->sc->lvl), s));  // (norm_finish; the cycles keep it up)
   FB_CUDA(cudaEventRecord(m->ev0, s));
   if (perm) {
     FB_TRY(perm_to_lattice(m, m->bb, rhs, perm, n));
@@ -2320,6 +2321,7 @@ int fb_mg_vcycle(fb_mg* m, const double* def, double* cor) {
   FB_TRY(ensure_vectors(m, m->cfg.precision));
   const uint32_t n = m->L[0].n;
   cudaStream_t s = m->stream;
+  FB_CUDA(cudaMemsetAsync(m->sc->lvl, 0, sizeof(m->sc->lvl), s));  // (norm_finish)
   if (m->feat_dof) FB_TRY(perm_to_lattice(m, m->r, def, m->feat_dof, n));
   else FB_CUDA(cudaMemcpyAsync(m->r, def, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
   k_dot_rz<double><<<occupancy_grid((const void*)k_dot_rz<double>, n / 32 + 1), 256, 0, s>>>(m->r, m->r, n, m->ws, m->counter, &m->sc->rr);

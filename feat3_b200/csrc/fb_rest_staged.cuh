@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(288, 1) k_rest_q1_staged(MfTile G, uint32_t Mf
   }
   pdl_trigger();
   const double blk = block_sum<288>(acc, sh);
-  reduce_finish<288>(blk, ws, counter, red_out, sh, false);
+  epi_finish<288>(epi, blk, ws, counter, red_out, sh);
 }
 
 }  // namespace fb

@@ -80,6 +80,43 @@ __device__ __forceinline__ bool smoother_skip(const double* sumsq) {
   return !(isfinite(nrm)) || nrm <= e * e;
 }
 
+// ------------------------------------------------------------------ finish of an epilogue's sum
+// A level's norms (the restricted right-hand side's and the first post-smoothing defect's) only feed
+// the smoothers' skip test, which compares them with eps^2: their block partials are added to the
+// level's scalar without waiting for the result. The ordered finish (reduce_finish: a memory fence, a
+// counter and the last block's second pass) cost each of these launches about 2 us of latency: 2D Q1
+// 129^2 FP64 solve 483 against 527 us, 513^2 solve and adjoint 4.80 against 5.63 ms, 129^3 mixed
+// matrix-free solve 3.19 against 3.41 ms, 257^3 13.86 against 14.13 ms. The other sums, which enter the iterates or are returned, keep it. The scalar starts from zero: the
+// restriction from a level clears that level's defect norm (`clear`), whose readers are done, and the
+// first post-smoothing step of a level clears the next coarser level's right-hand-side norm.
+template<typename Epi, typename = void> struct IsNorm { static constexpr bool value = false; };
+template<typename Epi> struct IsNorm<Epi, typename std::enable_if<Epi::kNorm>::type> { static constexpr bool value = true; };
+
+__device__ __forceinline__ void norm_finish(double blk, double* out, double* clear, bool first) {
+  atomicAdd(out, blk);
+  if (first && clear) *clear = 0.0;
+}
+
+template<int THREADS, typename Epi>
+__device__ __forceinline__ void epi_finish(const Epi& epi, double blk, double* ws, unsigned* counter, double* out, double* sh) {
+  if constexpr (IsNorm<Epi>::value) {
+    if (threadIdx.x == 0) norm_finish(blk, out, epi.clear, blockIdx.x == 0);
+  } else {
+    reduce_finish<THREADS>(blk, ws, counter, out, sh, false);
+  }
+}
+
+// the same for 2D/3D blocks and grids: tid = flattened thread, bid = linear block, nblk = blocks
+template<int THREADS, typename Epi>
+__device__ __forceinline__ void epi_finish_nd(const Epi& epi, double blk, double* ws, unsigned* counter, double* out, double* sh,
+                                              uint32_t tid, uint32_t bid, uint32_t nblk) {
+  if constexpr (IsNorm<Epi>::value) {
+    if (tid == 0) norm_finish(blk, out, epi.clear, bid == 0);
+  } else {
+    reduce_finish_nd<THREADS>(blk, ws, counter, out, sh, bid, nblk);
+  }
+}
+
 // ------------------------------------------------------------------ epilogues
 // r = a*s + b*y
 template<typename T>
@@ -114,8 +151,9 @@ struct EpiDefect {
 template<typename T, bool RED, bool DOT = false>
 struct EpiJacobi {
   static constexpr bool kReduce = RED || DOT;
+  static constexpr bool kNorm = RED;  // (norm_finish)
   const T* x; const T* rhs; const T* invd; T* out; const T* s0; const uint32_t* mask;
-  const double* skip_src; T omega;
+  const double* skip_src; T omega; double* clear = nullptr;
   __device__ __forceinline__ double operator()(uint32_t row, T s) const {
     // every input is loaded before out is stored (a load after the store would wait behind it)
     const T b = rhs[row];
@@ -168,7 +206,8 @@ struct EpiPcgQ {
 template<typename T>
 struct EpiRestrict {
   static constexpr bool kReduce = true;
-  T* rhs; T* sol1; const T* invd; const uint32_t* mask; T omega;
+  static constexpr bool kNorm = true;
+  T* rhs; T* sol1; const T* invd; const uint32_t* mask; T omega; double* clear = nullptr;
   __device__ __forceinline__ double operator()(uint32_t row, T s) const {
     const bool m = masked(mask, row);
     const T v = m ? T(0) : s;
@@ -370,7 +409,7 @@ __global__ void __launch_bounds__(256, sell_ctas<VT>()) k_sell(const __grid_cons
   }
   if (Epi::kReduce) {
     const double blk = block_sum<256>(acc, sh);
-    reduce_finish<256>(blk, ws, counter, red_out, sh, false);
+    epi_finish<256>(epi, blk, ws, counter, red_out, sh);
   }
 }
 
@@ -431,7 +470,7 @@ __global__ void __launch_bounds__(256) k_csr_epi(CsrView A, const XT* __restrict
   }
   if (Epi::kReduce) {
     const double blk = block_sum<256>(acc, sh);
-    reduce_finish<256>(blk, ws, counter, red_out, sh, false);
+    epi_finish<256>(epi, blk, ws, counter, red_out, sh);
   }
 }
 
@@ -512,7 +551,7 @@ __global__ void __launch_bounds__(256) k_stencil(StencilView<S> A, const XT* __r
   }
   if (Epi::kReduce) {
     const double blk = block_sum<256>(acc, sh);
-    reduce_finish<256>(blk, ws, counter, red_out, sh, false);
+    epi_finish<256>(epi, blk, ws, counter, red_out, sh);
   }
 }
 
@@ -609,7 +648,7 @@ __global__ void __launch_bounds__(256, 4) k_stencil_packed(StencilView<S> A, con
   }
   if (Epi::kReduce) {
     const double blk = block_sum<256>(acc, sh);
-    reduce_finish<256>(blk, ws, counter, red_out, sh, false);
+    epi_finish<256>(epi, blk, ws, counter, red_out, sh);
   }
 }
 
@@ -704,7 +743,7 @@ __global__ void __launch_bounds__(256) k_mf_q1(MfView<T, DIM> A, const T* __rest
   }
   if (Epi::kReduce) {
     const double blk = block_sum<256>(acc, sh);
-    reduce_finish<256>(blk, ws, counter, red_out, sh, false);
+    epi_finish<256>(epi, blk, ws, counter, red_out, sh);
   }
 }
 
@@ -820,7 +859,7 @@ __global__ void __launch_bounds__(256) k_rest_q1(Q1Transfer g, const T* __restri
     const double blk = block_sum_tid<256>(acc, sh, tid);
     const uint32_t nblk = gridDim.x * gridDim.y * gridDim.z;
     const uint32_t bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    reduce_finish_nd<256>(blk, ws, counter, red_out, sh, bid, nblk);
+    epi_finish_nd<256>(epi, blk, ws, counter, red_out, sh, tid, bid, nblk);
   }
 }
 
@@ -928,7 +967,7 @@ __global__ void __launch_bounds__(256) k_rest_q1_tile(Q1Transfer g, const T* __r
   const double blk = block_sum<256>(acc, sh);
   const uint32_t nblk = gridDim.x * gridDim.y * gridDim.z;
   const uint32_t bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  reduce_finish_nd<256>(blk, ws, counter, red_out, sh, bid, nblk);
+  epi_finish_nd<256>(epi, blk, ws, counter, red_out, sh, threadIdx.x, bid, nblk);
 }
 
 // 3D prolongation + coarse-grid correction with the coarse block in shared memory: a block

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(32 * (NCW + 1), 1)
   pdl_trigger();
   if (Epi::kReduce) {
     const double blk = block_sum<NT>(acc, sh);
-    reduce_finish<NT>(blk, ws, counter, red_out, sh, false);
+    epi_finish<NT>(epi, blk, ws, counter, red_out, sh);
   }
 }
 
