@@ -1120,6 +1120,10 @@ static int coarse_start(fb_mg* m) {
   const int nl = last_level(m) + 1;
   if (m->cfg.format != FB_FORMAT_MATFREE || m->cfg.coarse == FB_COARSE_PCG || (m->cfg.flags & FB_FLAG_NO_COARSE_FUSION))
     return nl;
+  // in 2D with a dense small end one level (65^2 points) is left to fuse, and its separate launches
+  // are faster: 513^2 solve and adjoint 5.63 against 5.87 ms, 1025^2 FP64 solve 6.25 against 6.43 ms
+  // (3D, 17^3 points: 33^3 solve 0.97 ms fused against 1.00, 257^3 mixed 14.25 against 14.30 ms)
+  if (m->dim == 2 && m->dense_l > 0) return nl;
   int lc = nl;
   for (int l = nl - 1; l >= 1; --l) {
     if (!m->L[l].mf || m->L[l].n > kCoarseRows) break;
