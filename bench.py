@@ -70,7 +70,7 @@ def workload(level):
                         f"f=1, Dirichlet 0; PCG + MG V(2,2) Richardson-Jacobi(0.5), levels 1..{level}, direct coarse",
             "dofs": n, "level": level,
             "l2": "inputs larger than L2 (126 MB): a finest-level matrix-free FP32 smoothing step streams 273 MB "
-                  "(x, k, rhs, result) at level 8; the assembled FP64 matrix is 5.5 GB"}
+                  "(x, k, rhs, result) at level 8; the assembled FP64 values are 3.7 GB"}
 
 
 def bench_config(args, world):
@@ -382,7 +382,7 @@ def native_arm(args):
             mat = ne * (8 if which == 3 else sx)          # per-cell coefficient instead of a matrix
         else:
             sv = {"f64": 8, "f32": 4, "f16": 2}[prec]
-            mat = nnz * (sv + (4 if fmt == "sell" else 0))  # values (+ 32-bit column indices)
+            mat = nnz * sv                                # values (the SELL chunks' columns are offset patterns)
         alg = mat + n * sx + vec + n / 8                  # + the input vector once + the filter mask
         rf[name] = {"ms": ms.value, "bytes": alg, "GBps": alg / (ms.value * 1e-3) / 1e9}
     peaks = {}

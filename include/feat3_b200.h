@@ -251,8 +251,9 @@ FB_API void fb_mg_destroy(fb_mg* mg);
 #define FB_PREC_F32 1
 #define FB_PREC_F16 2
 /* level-matrix storage of the V-cycle and the outer solver:
- *   FB_FORMAT_SELL    SELL-C-sigma with 32-bit column indices and CSR transfer matrices
- *                     (what a hierarchy handed over by FEAT3 uses);
+ *   FB_FORMAT_SELL    SELL-C-sigma with 32-bit column indices (offset patterns where the rows of a
+ *                     chunk share them) and CSR transfer matrices (what a hierarchy handed over by
+ *                     FEAT3 uses);
  *   FB_FORMAT_STENCIL on structured Q1 hierarchies: SELL-32 with implicit stencil columns
  *                     (no index stream) and matrix-free Q1 interpolation/restriction;
  *                     other hierarchies fall back to FB_FORMAT_SELL level by level;
