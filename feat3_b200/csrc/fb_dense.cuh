@@ -9,7 +9,7 @@
 // which costs its latency (2-4 us) for a few KB of work.
 // Whole solves with / without it: 2D Q1 129^2 FP64 V(4,4) 0.65 / 1.19 ms, 65^3 FP64 handed over as CSR
 // 3.55 / 4.29 ms, 2D Q2 1025^2 on FP16 values 19.2 / 22.3 ms, 257^3 mixed matrix-free 14.13 / 14.40 ms
-// (its coarse cluster then runs one level instead of four); it adds 0.7 ms to the configuration. In the
+// (its coarse cluster then runs one level instead of four); it adds 0.3-0.4 ms to the configuration. In the
 // FP32 and FP16 forms these levels' matrices enter in FP64 and only the operator is rounded.
 #pragma once
 #include "fb_sell.cuh"
@@ -38,11 +38,15 @@ struct DenseArgs {
 };
 
 // The columns col0 .. col0 + NC - 1 of the operator: the cycle on NC unit vectors, one CTA, all
-// vectors in shared memory ([level][rhs, x, y][row][NC]).
+// vectors in shared memory ([level][rhs, x, y][row][NC]); op is zero before the launch.
 template<typename T, int NC>
 __global__ void __launch_bounds__(kDenseThreads) k_dense_build(DenseArgs D, T* op, uint32_t ld) {
   extern __shared__ double dsm[];
   const uint32_t col0 = blockIdx.x * NC, tid = threadIdx.x;
+  // a Dirichlet entry's column stays zero (half of the 9^3 level's)
+  bool inner = false;
+  for (uint32_t c = col0; c < col0 + NC && c < D.L[0].n; ++c) inner = inner || !masked(D.L[0].mask, c);
+  if (!inner) return;
   const double om = D.omega;
   double* rhs[kDenseMax];
   double* xs[kDenseMax];
