@@ -1023,9 +1023,10 @@ static int last_solver(const fb_mg* m) { return m->dense_l > 0 ? FB_COARSE_DIREC
 template<typename T>
 static int launch_dense(fb_mg* m, int l, const T* b) {
   Level& L = m->L[l];
-  const bool op = l == m->dense_l;
+  const bool op = m->dense_l > 0 && l == m->dense_l;  // (0 = none: a one-level hierarchy's level 0 has the inverse)
   const T* a;
   if constexpr (std::is_same<T, double>::value) a = op ? m->dop64 : m->cinv64; else a = op ? m->dop32 : m->cinv32;
+  if (!a) return FB_ERR_NOT_READY;
   const uint32_t ld = dense_ld(L.n);
   FB_CUDA(launch_pdl(m->stream, k_dense_solve<T>, dim3(grid_for(L.n, 4)), dim3(128), ld * sizeof(T), Prec<T>::x(L), a, ld, b,
                      L.n));
