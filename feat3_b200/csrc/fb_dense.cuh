@@ -2,8 +2,8 @@
 //
 // From the first level of at most kDenseRows rows downwards, the cycle maps the level's right-hand
 // side to its correction by a fixed linear operator (damped Jacobi steps, transfers and the direct,
-// smoothing or identity coarse solver are linear; the smoothers' skip test only ever replaces the
-// step by zero for a right-hand side that is itself zero to rounding, or not finite). k_dense_build
+// smoothing or identity coarse solver are linear; the smoothers' skip test, which is absolute, is not, so
+// cycles on defects that it could act on run level by level: dense_applies in fb_mg.cu). k_dense_build
 // forms it column by column in FP64 when the solver is configured; a cycle then applies it as one
 // matrix-vector product (dense_rows) in place of some 2 nu + 3 dependent launches per level, each of
 // which costs its latency (2-4 us) for a few KB of work.

@@ -1015,15 +1015,32 @@ static int presmooth(fb_mg* m, int l, const T* b, const double* bnorm, bool need
 }
 
 // ------------------------------------------------------------------ dense small end
+// the level of the dense operator in the cycle being issued, 0 = none
+static int dense_level(const fb_mg* m) { return m->dense_on ? m->dense_l : 0; }
 // The V-cycle's last level and its solver: the level of the dense operator when one was built
 // (build_dense), else the coarsest level with the configured coarse solver.
-static int last_level(const fb_mg* m) { return m->dense_l > 0 ? m->dense_l : (int)m->L.size() - 1; }
-static int last_solver(const fb_mg* m) { return m->dense_l > 0 ? FB_COARSE_DIRECT : m->cfg.coarse; }
+static int last_level(const fb_mg* m) { return dense_level(m) > 0 ? dense_level(m) : (int)m->L.size() - 1; }
+static int last_solver(const fb_mg* m) { return dense_level(m) > 0 ? FB_COARSE_DIRECT : m->cfg.coarse; }
+
+// Whether a cycle on a defect of norm d (finest level) may use the dense operator. The operator holds
+// no skip test (smoother_skip), and the test is absolute: a level's smoother is left out where its
+// right-hand side or defect is at most eps^2 (1.4e-14 in FP32) or not finite. The norms on the small
+// levels scale with d; in PCG solves of 2D Q1, 2D Q2 and 3D Q1 problems those of the levels that
+// smooth were typically above 1e-3 d (the smallest on 25 rows). So above 1024 eps^2 the test would not
+// act, or only on parts a thousand times smaller than the cycle; the upper bounds keep every sum of
+// squares finite. All other cycles run level by level, with the tests. Tiny defects are met at the end of
+// FP32 solves: the 257^3 mixed solve runs its last two iterations level by level, 13.71 -> 13.77 ms.
+static bool dense_applies(const fb_mg* m, double d) {
+  if (m->dense_l == 0) return true;
+  const bool low = m->cfg.precision != FB_PREC_F64;
+  const double e = low ? double(eps_of<float>()) : eps_of<double>();
+  return d > 1024.0 * e * e && d < (low ? 3e32 : 1e148);
+}
 
 template<typename T>
 static int launch_dense(fb_mg* m, int l, const T* b) {
   Level& L = m->L[l];
-  const bool op = m->dense_l > 0 && l == m->dense_l;  // (0 = none: a one-level hierarchy's level 0 has the inverse)
+  const bool op = l > 0 && l == dense_level(m);  // (a one-level hierarchy's level 0 has the inverse)
   const T* a;
   if constexpr (std::is_same<T, double>::value) a = op ? m->dop64 : m->cinv64; else a = op ? m->dop32 : m->cinv32;
   if (!a) return FB_ERR_NOT_READY;
@@ -1124,7 +1141,7 @@ static int coarse_start(fb_mg* m) {
   // in 2D with a dense small end one level (65^2 points) is left to fuse, and its separate launches
   // are faster: 513^2 solve and adjoint 5.63 against 5.87 ms, 1025^2 FP64 solve 6.25 against 6.43 ms
   // (3D, 17^3 points: 33^3 solve 0.97 ms fused against 1.00, 257^3 mixed 14.25 against 14.30 ms)
-  if (m->dim == 2 && m->dense_l > 0) return nl;
+  if (m->dim == 2 && dense_level(m) > 0) return nl;
   int lc = nl;
   for (int l = nl - 1; l >= 1; --l) {
     if (!m->L[l].mf || m->L[l].n > kCoarseRows) break;
@@ -1144,7 +1161,7 @@ static int launch_coarse(fb_mg* m, int lc, T** sol_lc) {
   A.nu = m->cfg.nu;
   A.coarse = last_solver(m);
   A.omega = T(m->cfg.omega_rich);
-  const bool op = m->dense_l > 0;
+  const bool op = dense_level(m) > 0;
   if constexpr (std::is_same<T, double>::value) A.cinv = op ? m->dop64 : m->cinv64; else A.cinv = op ? m->dop32 : m->cinv32;
   A.ldc = dense_ld(m->L[nl - 1].n);
   A.s1_coarsest = A.coarse == FB_COARSE_SMOOTHER ? 1 : 0;
@@ -1605,7 +1622,8 @@ static int body(fb_mg* m, int j) {
 }
 
 static int run_body(fb_mg* m, int j) {
-  if (!m->cfg.use_graphs || debug_enabled()) return body(m, j);
+  // (the rare cycles without the dense operator are not captured)
+  if (!m->cfg.use_graphs || debug_enabled() || !m->dense_on) return body(m, j);
   // one graph per parity of j (the direction buffers alternate)
   const int par = j & 1;
   const int key = ((m->cfg.cycle * 4 + m->cfg.adapt_cgc) * 16 + m->cfg.flags) * 256 + m->cfg.format * 64 +
@@ -2141,7 +2159,10 @@ int solve_dev(fb_mg* m, const double* rhs, double* sol, double* hist, fb_solve_i
   // a staged kernel whose bounded wait expired has left rows unwritten: the solve stops at the
   // next read-back and returns FB_ERR_TIMEOUT (check_kernel_waits below)
   while (status == 1 && !host_kerr(m)) {
-    FB_TRY(run_body(m, it + 1));
+    m->dense_on = dense_applies(m, d);
+    const int rc = run_body(m, it + 1);
+    m->dense_on = true;
+    FB_TRY(rc);
     FB_CUDA(cudaStreamSynchronize(s));
     ++it;
     d = std::sqrt(*m->host_rr);
@@ -2331,23 +2352,34 @@ int fb_mg_vcycle(fb_mg* m, const double* def, double* cor) {
   else FB_CUDA(cudaMemcpyAsync(m->r, def, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
   k_dot_rz<double><<<occupancy_grid((const void*)k_dot_rz<double>, n / 32 + 1), 256, 0, s>>>(m->r, m->r, n, m->ws, m->counter, &m->sc->rr);
   FB_CHECK_LAUNCH();
-  const void* z = nullptr;
   if (m->cfg.precision != FB_PREC_F64) {
     k_cvt<float, double><<<ew_grid(n), 256, 0, s>>>(m->r32, m->r, n);
     FB_CHECK_LAUNCH();
   }
-  FB_TRY(precond(m, &z));
-  double* out = cor;
-  if (m->feat_dof) {
-    if (!m->pv1) FB_TRY(dalloc(m, &m->pv1, n));
-    out = m->pv1;
-  }
-  if (m->cfg.precision == FB_PREC_F64) FB_CUDA(cudaMemcpyAsync(out, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  else { k_cvt<double, float><<<ew_grid(n), 256, 0, s>>>(out, (const float*)z, n); FB_CHECK_LAUNCH(); }
-  if (m->feat_dof) FB_TRY(perm_from_lattice(m, cor, out, m->feat_dof, n));
-  FB_CUDA(cudaStreamSynchronize(s));
+  if (m->feat_dof && !m->pv1) FB_TRY(dalloc(m, &m->pv1, n));
+  // from m->r to cor; the defect's norm and the wait flag come to the host behind it
+  auto cycle = [&]() -> int {
+    const void* z = nullptr;
+    FB_TRY(precond(m, &z));
+    double* out = m->feat_dof ? m->pv1 : cor;
+    if (m->cfg.precision == FB_PREC_F64) FB_CUDA(cudaMemcpyAsync(out, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    else { k_cvt<double, float><<<ew_grid(n), 256, 0, s>>>(out, (const float*)z, n); FB_CHECK_LAUNCH(); }
+    if (m->feat_dof) FB_TRY(perm_from_lattice(m, cor, out, m->feat_dof, n));
+    FB_CUDA(cudaMemcpyAsync(m->host_rr, &m->sc->rr, kHostScalarBytes, cudaMemcpyDeviceToHost, s));
+    FB_CUDA(cudaStreamSynchronize(s));
+    return FB_OK;
+  };
+  FB_TRY(cycle());
   // a staged kernel whose bounded wait expired left rows unwritten: FB_ERR_TIMEOUT
-  return check_kernel_waits(m);
+  if (host_kerr(m)) return check_kernel_waits(m);
+  if (dense_applies(m, std::sqrt(*m->host_rr))) return FB_OK;
+  // the norm is known only now: once more, level by level
+  FB_CUDA(cudaMemsetAsync(m->sc->lvl, 0, sizeof(m->sc->lvl), s));
+  m->dense_on = false;
+  const int rc = cycle();
+  m->dense_on = true;
+  FB_TRY(rc);
+  return host_kerr(m) ? check_kernel_waits(m) : FB_OK;
 }
 
 int fb_mg_test_expire_wait(fb_mg* m) {

@@ -141,8 +141,10 @@ struct fb_mg {
   uint32_t nc = 0;
   double* cinv64 = nullptr;
   float* cinv32 = nullptr;       // (rows of dense_ld(nc))
-  // the small end of the V-cycle as a dense operator (fb_dense.cuh): its level, 0 = none
+  // the small end of the V-cycle as a dense operator (fb_dense.cuh): its level, 0 = none, and whether
+  // the cycle being issued uses it (dense_applies)
   int dense_l = 0;
+  bool dense_on = true;
   double* dop64 = nullptr;
   float* dop32 = nullptr;
   // outer (finest) vectors

@@ -65,3 +65,42 @@ def test_handed_hierarchy_matches_oracle(sigma):
     mg = MultiGrid.from_csr(levels, sell_sigma=sigma).configure(nu=3)
     assert relerr(mg.vcycle(torch.tensor(d).cuda()).cpu().numpy(), H.vcycle(d, nu=3)) <= 1e-13
     mg.close()
+
+
+TINY = [(2, 1, 7, 1, 2, "direct"), (2, 1, 6, 2, 3, "smoother"), (3, 1, 5, 1, 2, "direct"), (2, 2, 5, 1, 1, "none")]
+
+
+@pytest.mark.parametrize("fmt", ["sell", "matfree"])
+@pytest.mark.parametrize("case", TINY, ids=["d%dq%dL%d-%d-nu%d-%s" % c for c in TINY])
+def test_tiny_and_non_finite_defects(case, fmt):
+    """the operator holds no skip test: a cycle on a defect that could meet one runs level by level"""
+    from feat3_b200.solver import MultiGrid
+    dim, deg, lvl, lmin, nu, coarse = case
+    k = coefficient(dim, lvl)
+    H = po.Hierarchy(dim, deg, lvl, lmin, k)
+    d = H.rhs("one") * np.random.default_rng(6).uniform(0.5, 1.5, H.ndofs())
+    d /= np.linalg.norm(d)
+    mg = MultiGrid.structured(dim, deg, lvl, lmin, k)
+    for prec, eps, tol in (("f64", 2.0 ** -52, 1e-13), ("f32", 2.0 ** -23, 6e-6)):
+        mg.configure(nu=nu, coarse=coarse, precision=prec, format=fmt)
+        plain = mg.vcycle(torch.tensor(d).cuda()).cpu().numpy()
+        for size in (1e-3, 0.3, 3.0, 30.0, 1e9):  # norms in units of the skip test's eps^2
+            t = d * (size * eps ** 2)
+            out = mg.vcycle(torch.tensor(t).cuda()).cpu().numpy()
+            ref = H.vcycle(t, nu=nu, coarse=coarse, inner=prec)  # (zero where every smoother is left out)
+            assert np.linalg.norm(out - ref) <= tol * np.linalg.norm(ref), (prec, size)
+        np.testing.assert_array_equal(mg.vcycle(torch.tensor(d).cuda()).cpu().numpy(), plain)
+        # iterations of a solve whose small levels meet the test
+        t = d * (900.0 * eps ** 2)
+        out = mg.configure(nu=nu, coarse=coarse, precision=prec, format=fmt, max_iter=2).solve(torch.tensor(t).cuda())
+        ref = H.solve(t, nu=nu, coarse=coarse, inner=prec, max_iter=2)
+        np.testing.assert_allclose(out["hist"], ref["hist"], rtol=1e-4 if prec == "f32" else 1e-10)
+        if coarse == "smoother":
+            for bad in (np.inf, np.nan):
+                t = d.copy()
+                t[t.size // 2 + 3] = bad
+                mg.configure(nu=nu, coarse=coarse, precision=prec, format=fmt)
+                with np.errstate(invalid="ignore"):
+                    ref = H.vcycle(t, nu=nu, coarse=coarse, inner=prec)
+                np.testing.assert_array_equal(mg.vcycle(torch.tensor(t).cuda()).cpu().numpy(), ref)
+    mg.close()
