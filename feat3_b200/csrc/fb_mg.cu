@@ -570,9 +570,14 @@ __global__ void k_quant16_sell(__half* d, const double* __restrict__ s, double i
     for (uint32_t j = 0; j < len; ++j) {
       const uint32_t src = beg + j * 32u + lane;
       const uint32_t dst = j < even ? beg + (j >> 1) * 64u + 2u * lane + (j & 1u) : src;
-      d[dst] = __double2half(s[src] * inv);
+      d[dst] = sell_cvt(s[src] * inv, d);
     }
   }
+}
+
+__global__ void k_f32_sell(float* d, const double* __restrict__ s, uint64_t n) {
+  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
+    d[i] = sell_cvt(s[i], d);
 }
 
 unsigned ew_grid(uint64_t n) {
@@ -1654,10 +1659,10 @@ static int run_body(fb_mg* m, int j) {
 // A chunk follows a pattern when lane r's column in slot j is (slot row of r) + offset[j]: a row
 // with an entry in every slot (the reference lane) sets the offsets, and every other row's entries
 // follow them in the same order, with gaps (a lattice row next to the boundary, a Q2 edge row
-// between vertex rows). The row's entries move to the slots they match and the gaps hold value 0
-// (column ~0u in the 32-bit array, the mark of an empty slot). Every slot row + offset is a valid
-// column for all 32 lanes. The products and their order are those of the plain form (plus 0 * x of a
-// neighbouring column in the gaps).
+// between vertex rows). The row's entries move to the slots they match and the gaps hold value -0.0
+// (column ~0u in the 32-bit array, the mark of an empty slot); a chunk with gaps and an entry of -0.0
+// stays plain. Every slot row + offset is a valid column for all 32 lanes. The products and their order
+// are those of the plain form.
 struct SellSetup {
   uint32_t rows, cols, nchunks;
   const uint32_t *cs, *cl, *rl, *perm;
@@ -1684,6 +1689,10 @@ __global__ void __launch_bounds__(256) k_sell_candidates(SellSetup S) {
       ok = __all_sync(0xffffffffu, mine >= 0 && mine < int64_t(S.cols));
     }
     ok = __all_sync(0xffffffffu, ok && k == mylen);
+    if (ok && __any_sync(0xffffffffu, mylen < len)) {
+      for (k = 0; k < mylen; ++k) ok = ok && !sell_gap(S.val[e0 + k * 32u + lane]);
+      ok = __all_sync(0xffffffffu, ok);
+    }
     if (lane == 0) S.md[c] = ok ? len | uint32_t(ref + 1) << 23 : 0u;
   }
 }
@@ -1745,17 +1754,17 @@ __global__ void __launch_bounds__(256) k_sell_forms(SellSetup S) {
       for (int p = 0; p < kSellPatterns && !form; ++p)
         if (sell_follows(S, S.pat + p * kSellPatternSlots, S.plen[p], off, len, lane)) form = p + 1;
     }
+    const uint32_t mylen = sr < S.rows ? S.rl[S.perm ? S.perm[sr] : sr] : 0u;
     __syncwarp();
     if (lane == 0) S.md[c] = len | (form << 28);
     if (!form) continue;
-    const uint32_t mylen = sr < S.rows ? S.rl[S.perm ? S.perm[sr] : sr] : 0u;
     uint32_t* cp = S.col + e0 + lane;
     double* vp = S.val + e0 + lane;
     uint32_t k = mylen;  // from the last slot down: an entry only moves to a slot at or behind its own
     for (uint32_t j = len; j-- > 0;) {
       const uint32_t at = sr + uint32_t(S.pat[(form - 1) * kSellPatternSlots + j]);
       const bool here = k > 0 && cp[(k - 1u) * 32u] == at;
-      const double v = here ? vp[(k - 1u) * 32u] : 0.0;
+      const double v = here ? vp[(k - 1u) * 32u] : -0.0;
       if (here) --k;
       cp[j * 32u] = here ? at : 0xffffffffu;
       vp[j * 32u] = v;
@@ -1867,7 +1876,7 @@ static int ensure_vectors(fb_mg* m, int prec) {
       }
       if (need_sell && prec == FB_PREC_F32 && !L.A.v32) {
         FB_TRY(dalloc(m, &L.A.v32, L.A.nent));
-        k_cvt<float, double><<<ew_grid(L.A.nent), 256, 0, m->stream>>>(L.A.v32, L.A.v64, L.A.nent);
+        k_f32_sell<<<ew_grid(L.A.nent), 256, 0, m->stream>>>(L.A.v32, L.A.v64, L.A.nent);
         FB_CHECK_LAUNCH();
       }
       if (need_sell && prec == FB_PREC_F16 && !L.A.v16) {

@@ -9,7 +9,9 @@
 //
 // A chunk whose 32 rows have their columns at the same offsets from the row (lattice matrices)
 // refers to one of a few offset patterns, which are kernel parameters, and reads no column
-// indices; the others read a 32-bit column per entry (k_sell_forms finds the patterns).
+// indices; the others read a 32-bit column per entry (k_sell_forms finds the patterns). Where a row
+// lacks an entry of its chunk's pattern the slot holds -0.0, which no entry there does, and is left out
+// of the sum: an infinite or undefined x reaches only the rows that couple to it.
 #pragma once
 #include "fb_common.cuh"
 
@@ -118,6 +120,10 @@ __device__ __forceinline__ void epi_finish_nd(const Epi& epi, double blk, double
 }
 
 // ------------------------------------------------------------------ epilogues
+template<typename Epi> struct IsJacobi { static constexpr bool value = false; };
+template<typename T, bool RED, bool DOT = false> struct EpiJacobi;
+template<typename T, bool RED, bool DOT> struct IsJacobi<EpiJacobi<T, RED, DOT>> { static constexpr bool value = true; };
+
 // r = a*s + b*y
 template<typename T>
 struct EpiAxpby {
@@ -148,7 +154,7 @@ struct EpiDefect {
 // reduction: RED: ||filter_def(rhs - A x)||^2 (initial defect of the smoother, post-smoothing);
 // DOT: out . rhs (the last post-smoothing step of the finest level, whose result is the
 // preconditioned defect z and whose rhs is the outer defect r: PCG's r . z)
-template<typename T, bool RED, bool DOT = false>
+template<typename T, bool RED, bool DOT>
 struct EpiJacobi {
   static constexpr bool kReduce = RED || DOT;
   static constexpr bool kNorm = RED;  // (norm_finish)
@@ -321,8 +327,20 @@ struct EpiFiltered {
 };
 
 // ------------------------------------------------------------------ SELL kernel
-// adds the products of U slots from slot j on: the loads of all of them, then the sum in slot order
-template<int U, bool PAT, typename VT, typename XT, typename AT>
+// an empty slot of a chunk that follows a pattern
+__device__ __forceinline__ bool sell_gap(double v) { return __double_as_longlong(v) == __double_as_longlong(-0.0); }
+__device__ __forceinline__ bool sell_gap(float v) { return __float_as_uint(v) == 0x80000000u; }
+// a smaller type's copy of a value: an entry that underflows becomes +0, not an empty slot
+__device__ __forceinline__ float sell_cvt(double v, float*) { const float f = float(v); return f == 0.0f && v != 0.0 ? 0.0f : f; }
+__device__ __forceinline__ __half sell_cvt(double v, __half*) {
+  const __half h = __double2half(v);
+  return __half2float(h) == 0.0f && v != 0.0 ? __float2half(0.0f) : h;
+}
+
+// adds the products of U slots from slot j on: the loads of all of them, then the sum in slot order. An
+// empty slot of a pattern (PAT) is left out by a predicate on its product, or (SEL) by 0 in the place of
+// its x, -0.0 * 0 being no change: the faster of the two as measured (k_sell).
+template<int U, bool PAT, bool SEL, typename VT, typename XT, typename AT>
 __device__ __forceinline__ void sell_group(AT& sum, const uint32_t* __restrict__ col, const int32_t* pat,
                                            const VT* __restrict__ val, const VT* __restrict__ vpair,
                                            const XT* __restrict__ x, uint32_t srow, uint32_t j) {
@@ -346,12 +364,16 @@ __device__ __forceinline__ void sell_group(AT& sum, const uint32_t* __restrict__
 #pragma unroll
   for (int u = 0; u < U; ++u) xx[u] = __ldg(x + cc[u]);
 #pragma unroll
-  for (int u = 0; u < U; ++u) sum += vv[u] * AT(xx[u]);
+  for (int u = 0; u < U; ++u) {
+    if (!PAT) sum += vv[u] * AT(xx[u]);
+    else if (SEL) sum += vv[u] * (sell_gap(vv[u]) ? AT(0) : AT(xx[u]));
+    else if (!sell_gap(vv[u])) sum += vv[u] * AT(xx[u]);
+  }
 }
 
 // sum of a lane's products over its chunk's slots, in slot order; cs = the chunk's first entry,
-// srow = the lane's slot row, pat = the chunk's offsets (PAT)
-template<typename VT, typename XT, typename AT, int U, bool PAT>
+// srow = the lane's slot row, pat = the chunk's offsets
+template<typename VT, typename XT, typename AT, int U, bool PAT, bool SEL>
 __device__ __forceinline__ AT sell_sum(const SellView& A, const int32_t* pat, const XT* __restrict__ x, uint32_t cs,
                                        uint32_t len, uint32_t srow, uint32_t lane) {
   const VT* __restrict__ v = static_cast<const VT*>(A.val) + cs + lane;
@@ -362,13 +384,13 @@ __device__ __forceinline__ AT sell_sum(const SellView& A, const int32_t* pat, co
   AT sum = AT(0);
   uint32_t j = 0;
   if constexpr (sizeof(VT) == 2) {
-    for (; j + U <= len; j += U) sell_group<U, PAT>(sum, col, pat, v, vp, x, srow, j);
-    for (; j + 2 <= len; j += 2) sell_group<2, PAT>(sum, col, pat, v, vp, x, srow, j);
+    for (; j + U <= len; j += U) sell_group<U, PAT, SEL>(sum, col, pat, v, vp, x, srow, j);
+    for (; j + 2 <= len; j += 2) sell_group<2, PAT, SEL>(sum, col, pat, v, vp, x, srow, j);
   } else {
-    for (; j + U <= len; j += U) sell_group<U, PAT>(sum, col, pat, v, vp, x, srow, j);
-    for (; j + 3 <= len; j += 3) sell_group<3, PAT>(sum, col, pat, v, vp, x, srow, j);
+    for (; j + U <= len; j += U) sell_group<U, PAT, SEL>(sum, col, pat, v, vp, x, srow, j);
+    for (; j + 3 <= len; j += 3) sell_group<3, PAT, SEL>(sum, col, pat, v, vp, x, srow, j);
   }
-  for (; j < len; ++j) sell_group<1, PAT>(sum, col, pat, v, vp, x, srow, j);
+  for (; j < len; ++j) sell_group<1, PAT, SEL>(sum, col, pat, v, vp, x, srow, j);
   return sum;
 }
 
@@ -377,9 +399,12 @@ __device__ __forceinline__ AT sell_sum(const SellView& A, const int32_t* pat, co
 // measured at 257^3, Jacobi step / defect / PCG-q: FP64 8 slots (9 for PCG-q) in at most 64
 // registers 649 / 617 / 619 us (32 registers 648 / 631 / 619, no bound 730 / 668 / 712); FP32 8 slots
 // in 32 registers 398 / 382 us (no bound 595 / 519); FP16 12 slots without a bound 359 / 314 us (8
-// slots 463 / 404, 14 slots in 32 registers 407 / 356). With a 32-bit column read per entry the same
-// steps took 909 / 889 / 874, 644 / 640 and 516 / 642 us. FP64 streams 4.2 GB per Jacobi step, 6.5
-// TB/s; FP32 and FP16 are bound by their x loads' issue, not by the bytes.
+// slots 463 / 404, 14 slots in 32 registers 407 / 356); these with the empty slots multiplied. With a
+// 32-bit column read per entry the same steps took 909 / 889 / 874, 644 / 640 and 516 / 642 us.
+// Empty slots left out: FP64 648 / 620 / 604 us (multiplied 649 / 618 / 597; the predicate in the Jacobi
+// step 673, the other form in the defect 637), FP32 404 / 386 (399 / 377), FP16 330 / 298 (366 / 319).
+// A third loop for the chunks with empty slots ran slower in FP64 (650 / 692 / 632). FP64 streams 4.2 GB
+// per Jacobi step, 6.5 TB/s; FP32 and FP16 are bound by their x loads' issue, not by the bytes.
 template<typename VT> constexpr int sell_ctas() { return sizeof(VT) == 8 ? 4 : (sizeof(VT) == 4 ? 8 : 1); }
 template<typename VT, typename XT, typename AT, typename Epi>
 __global__ void __launch_bounds__(256, sell_ctas<VT>()) k_sell(const __grid_constant__ SellView A, const XT* __restrict__ x, Epi epi,
@@ -388,6 +413,7 @@ __global__ void __launch_bounds__(256, sell_ctas<VT>()) k_sell(const __grid_cons
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t step = gridDim.x * (blockDim.x >> 5);
   constexpr int U = sizeof(VT) == 2 ? 12 : (std::is_same<Epi, EpiPcgQ<AT, XT>>::value ? 9 : 8);
+  constexpr bool SEL = sizeof(VT) == 8 && IsJacobi<Epi>::value;
   double acc = 0.0;
   uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   uint32_t cs = c < A.nchunks ? __ldg(A.cs + c) : 0u, md = c < A.nchunks ? __ldg(A.md + c) : 0u;
@@ -400,8 +426,8 @@ __global__ void __launch_bounds__(256, sell_ctas<VT>()) k_sell(const __grid_cons
       cs = __ldg(A.cs + c);
       md = __ldg(A.md + c);
     }
-    AT sum = form ? sell_sum<VT, XT, AT, U, true>(A, A.pat[form - 1], x, cs0, len, srow, lane)
-                  : sell_sum<VT, XT, AT, U, false>(A, nullptr, x, cs0, len, srow, lane);
+    AT sum = form ? sell_sum<VT, XT, AT, U, true, SEL>(A, A.pat[form - 1], x, cs0, len, srow, lane)
+                  : sell_sum<VT, XT, AT, U, false, SEL>(A, nullptr, x, cs0, len, srow, lane);
     if (srow < A.rows) {
       if (sizeof(VT) == 2) sum *= AT(A.scale);
       acc += epi(A.perm ? __ldg(A.perm + srow) : srow, sum);

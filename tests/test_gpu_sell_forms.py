@@ -106,3 +106,41 @@ def test_products(name, sigma):
     np.testing.assert_array_equal(eci, ci)
     np.testing.assert_array_equal(eva, va)
     mg.close()
+
+
+@pytest.mark.parametrize("prec", ["f32", "f16"])
+@pytest.mark.parametrize("name", ["q1_2d_70x67", "q1_3d_33", "q2_2d_65", "bands", "scattered"])
+def test_infinite_entry_reaches_coupled_rows_only(name, prec):
+    """two smoothing steps on a defect with one entry that overflows FP32: the second step's product
+    is not finite in the rows with an entry in that column (one of value -0.0 or that underflows
+    included) and in no other, wherever the rows of a pattern lack entries"""
+    from feat3_b200.solver import MultiGrid
+    rp, ci = CASES[name]()
+    n = rp.size - 1
+    rng = np.random.default_rng(11)
+    va = rng.uniform(0.1, 1.0, ci.size)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    off = ci != rows
+    va[off & (rng.random(ci.size) < 0.05)] = -1e-12  # (0 in FP16)
+    part = off & (rows < n // 3)                     # chunks with such entries, and chunks without
+    va[part & (rng.random(ci.size) < 0.01)] = -0.0
+    va[~off] = 4.0 + rng.uniform(0.0, 1.0, n)
+    A = sp.csr_matrix((va, ci, rp), shape=(n, n), copy=True)
+    w = 0.5 / A.diagonal()
+    b = rng.standard_normal(n)
+    mg = MultiGrid.from_csr([{"A": (rp, ci, va), "filter": np.zeros(0, np.int64)}])
+    mg.configure(nu=2, coarse="smoother", precision=prec)
+    shape = {"q1_2d_70x67": 70, "q1_3d_33": 33, "q2_2d_65": 65}.get(name, 64)
+    for c in (0, 1, shape - 1, shape, n // 2 - n // 2 % shape - 1, n // 2 - n // 2 % shape, n // 2 + 7, n - shape, n - 1):
+        d = b.copy()
+        d[c] = 1e39  # infinite in FP32; the norm in FP64 is finite, so the smoother runs
+        z = mg.vcycle(torch.tensor(d).cuda()).cpu().numpy()
+        coupled = np.zeros(n, bool)
+        coupled[rows[ci == c]] = True
+        np.testing.assert_array_equal(~np.isfinite(z), coupled)
+        s = w * b
+        ref = s + w * (b - A @ s)
+        e = {"f32": 2.0 ** -20, "f16": 2.0 ** -9}[prec]  # at most 41 additions, or the values' rounding
+        lim = e * (abs(s) + w * (abs(b) + abs(A) @ abs(s)))
+        assert np.all(abs(z - ref)[~coupled] <= lim[~coupled])
+    mg.close()
