@@ -450,11 +450,21 @@ struct CsrView {
 // Part of a CSR row's product by lane `sub` of the G that share the row: entries beg + sub,
 // beg + sub + G, ... in this order. The loads of four of them are issued together (past the row's
 // end: its last entry again, not summed), so a lane waits for memory twice per four entries.
+// A row that ends within four steps of the 32-bit limit, where a position past its end would wrap
+// around, is walked one entry at a time by its offset.
 template<int G, typename VT, typename XT, typename AT, typename IT>
 __device__ __forceinline__ AT csr_row(const VT* __restrict__ val, const IT* __restrict__ col, const XT* __restrict__ x,
                                       IT beg, IT end, int sub) {
   constexpr int U = 4;
   AT sum(0);
+  if (sizeof(IT) == 4 && end > IT(0) - IT((U + 1) * G)) {
+#pragma unroll 1
+    for (uint64_t o = sub; beg + o < end; o += G) {
+      const IT at = beg + IT(o);
+      sum += AT(ValLoad<VT>::ld(val + at)) * AT(__ldg(x + __ldg(col + at)));
+    }
+    return sum;
+  }
   for (IT k = beg + IT(sub); k < end; k += IT(U * G)) {
     IT cc[U];
     AT vv[U];

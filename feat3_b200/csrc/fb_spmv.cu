@@ -39,7 +39,13 @@ __global__ void k_csr_t(T* r, T a, const T* __restrict__ x, const T* __restrict_
   const int sub = threadIdx.x % 8;
   if (row >= rows) return;
   const T xa = a * x[row];
-  for (IT k = rp[row] + sub; k < rp[row + 1]; k += 8) atomicAdd(&r[col[k]], val[k] * xa);
+  const IT beg = rp[row], end = rp[row + 1];
+  if (beg >= end) return;
+  // (offsets from the row's start: a position past its end may lie behind the index type's limit)
+  for (uint64_t o = sub; o < uint64_t(end - beg); o += 8) {
+    const IT k = beg + IT(o);
+    atomicAdd(&r[col[k]], val[k] * xa);
+  }
 }
 
 // FEAT's SELL-C rows, one thread per row; the loads of eight slots are issued together (two memory

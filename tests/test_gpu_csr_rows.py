@@ -39,3 +39,36 @@ def test_rows(name, dtype, eps, index):
     bound = (rl + 3) * eps * (terms + abs(y))  # one rounding per entry, three for a, b and the sum
     assert np.all(abs(A.apply(R, X).numpy() - S @ x) <= bound)
     assert np.all(abs(A.apply(R, X, Y, -1.0).numpy() - (y - S @ x)) <= bound)
+
+
+@pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
+@pytest.mark.parametrize("avg", [3, 9, 16, 27, 50, 125])
+def test_last_row_at_the_index_limit(avg, dtype, eps):
+    """32-bit row pointers up to 2^32 - 1: a lane's next position would lie behind the limit. The
+    arrays start where the first of these rows does (their addresses are shifted by its position), and
+    the mean row length given picks the threads per row."""
+    from feat3_b200 import _lib
+    sfx = "f64" if dtype == torch.float64 else "f32"
+    rng = np.random.default_rng(avg)
+    m = 300
+    for rl in ([1, 2, 0, 5], [40, 127, 0, 130], [300, 1], [7]):
+        end = 2 ** 32 - 1
+        rp = end - sum(rl) + np.concatenate([[0], np.cumsum(rl)])
+        nnz, n = sum(rl), len(rl)
+        ci = np.concatenate([np.sort(rng.choice(m, k, replace=False)) for k in rl])
+        va = rng.standard_normal(nnz).astype(np.float32).astype(np.float64)
+        x = rng.standard_normal(max(m, n)).astype(np.float32).astype(np.float64)
+        S = sp.csr_matrix((va, ci, rp - rp[0]), shape=(n, m), copy=True)
+        dev = lambda a, t: torch.tensor(a, dtype=t).cuda()
+        V, X, Y, R = dev(va, dtype), dev(x, dtype), dev(np.zeros(m), dtype), dev(np.full(m, np.nan), dtype)
+        C = torch.tensor(ci.astype(np.uint32).view(np.int32)).cuda()
+        P = torch.tensor(rp.astype(np.uint32).view(np.int32)).cuda()
+        first = int(rp[0])
+        args = (V.data_ptr() - first * V.element_size(), C.data_ptr() - first * 4, P.data_ptr())
+        st = torch.cuda.current_stream().cuda_stream
+        _lib.call("fb_csr_apply_" + sfx, R.data_ptr(), 1.0, X.data_ptr(), 0.0, None, *args, n, m, avg * n, 0, st)
+        bound = (np.array(rl) + 3) * eps * (abs(S) @ abs(x[:m]))
+        assert np.all(abs(R[:n].double().cpu().numpy() - S @ x[:m]) <= bound)
+        _lib.call("fb_csr_apply_" + sfx, R.data_ptr(), 1.0, X.data_ptr(), 0.0, None, *args, n, m, avg * n, 1, st)
+        bound = (n + 3) * eps * (abs(S).T @ abs(x[:n]))
+        assert np.all(abs(R.double().cpu().numpy() - S.T @ x[:n]) <= bound)
