@@ -105,17 +105,19 @@ template<typename VT, typename XT, typename AT, typename Epi>
 static int launch_csr(fb_mg* m, const DevCsr& A, bool f32, const XT* x, const Epi& epi, double* red_out) {
   // threads per row: 1 for prolongations (3.4 entries a row in 3D), 4 for 2D restrictions, 8 for 3D
   // ones (27). A 129^3 FP32 cycle on SELL matrices takes 529 us so, 543 with 2 and 4 threads, 582
-  // with 4 and 16 (595 with these and one entry loaded at a time); a 1025^2 Q2 one 390, 390, 428 us
+  // with 4 and 16 (595 with these and one entry loaded at a time); a 1025^2 Q2 one 390, 390, 428 us. The
+  // sums per thread (csr_row) keep the terms in groups of 4, 8 and 16
   const double avg = A.rows ? double(A.nnz) / double(A.rows) : 0.0;
-  auto launch = [&](auto g) {
-    constexpr int G = decltype(g)::value;
-    auto fn = k_csr_epi<VT, XT, AT, Epi, G>;
+  auto launch = [&](auto g, auto p) {
+    constexpr int G = decltype(g)::value, P = decltype(p)::value;
+    auto fn = k_csr_epi<VT, XT, AT, Epi, G, P>;
     const int grid = occupancy_grid((const void*)fn, (uint64_t(A.rows) * G + 31) / 32);
     return launch_pdl(m->stream, fn, dim3(grid), dim3(256), 0, A.view(f32), x, epi, m->ws, m->counter, red_out);
   };
-  if (avg <= 4.0) FB_CUDA(launch(std::integral_constant<int, 1>()));
-  else if (avg <= 12.0) FB_CUDA(launch(std::integral_constant<int, 4>()));
-  else FB_CUDA(launch(std::integral_constant<int, 8>()));
+  using std::integral_constant;
+  if (avg <= 4.0) FB_CUDA(launch(integral_constant<int, 1>(), integral_constant<int, 4>()));
+  else if (avg <= 12.0) FB_CUDA(launch(integral_constant<int, 4>(), integral_constant<int, 2>()));
+  else FB_CUDA(launch(integral_constant<int, 8>(), integral_constant<int, 2>()));
   m->launches++;
   FB_CHECK_LAUNCH();
   return FB_OK;

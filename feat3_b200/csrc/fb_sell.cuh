@@ -449,15 +449,17 @@ struct CsrView {
 
 // Part of a CSR row's product by lane `sub` of the G that share the row: entries beg + sub,
 // beg + sub + G, ... in this order. The loads of four of them are issued together (past the row's
-// end: its last entry again, not summed), so a lane waits for memory twice per four entries.
+// end: its last entry again, not summed), so a lane waits for memory twice per four entries. P (1, 2 or
+// 4) sums per lane, taken in turn and added last: the terms are grouped, and rounded, as by P G lanes with
+// one sum each (figures in csr_apply, fb_spmv.cu).
 // A row that ends within four steps of the 32-bit limit, where a position past its end would wrap
 // around, is walked one entry at a time by its offset.
-template<int G, typename VT, typename XT, typename AT, typename IT>
+template<int G, int P, typename VT, typename XT, typename AT, typename IT>
 __device__ __forceinline__ AT csr_row(const VT* __restrict__ val, const IT* __restrict__ col, const XT* __restrict__ x,
                                       IT beg, IT end, int sub) {
   constexpr int U = 4;
-  AT sum(0);
   if (sizeof(IT) == 4 && end > IT(0) - IT((U + 1) * G)) {
+    AT sum(0);
 #pragma unroll 1
     for (uint64_t o = sub; beg + o < end; o += G) {
       const IT at = beg + IT(o);
@@ -465,6 +467,8 @@ __device__ __forceinline__ AT csr_row(const VT* __restrict__ val, const IT* __re
     }
     return sum;
   }
+  static_assert(P == 1 || P == 2 || P == 4, "sums per lane");
+  AT part[P] = {};
   for (IT k = beg + IT(sub); k < end; k += IT(U * G)) {
     IT cc[U];
     AT vv[U];
@@ -479,12 +483,14 @@ __device__ __forceinline__ AT csr_row(const VT* __restrict__ val, const IT* __re
     for (int u = 0; u < U; ++u) xx[u] = __ldg(x + cc[u]);
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (k + IT(u * G) < end) sum += vv[u] * AT(xx[u]);
+      if (k + IT(u * G) < end) part[u % P] += vv[u] * AT(xx[u]);
   }
-  return sum;
+  if constexpr (P == 4) return (part[0] + part[2]) + (part[1] + part[3]);
+  else if constexpr (P == 2) return part[0] + part[1];
+  else return part[0];
 }
 
-template<typename VT, typename XT, typename AT, typename Epi, int G>
+template<typename VT, typename XT, typename AT, typename Epi, int G, int P>
 __global__ void __launch_bounds__(256) k_csr_epi(CsrView A, const XT* __restrict__ x, Epi epi,
                                                  double* ws, unsigned* counter, double* red_out) {
   __shared__ double sh[8];
@@ -499,7 +505,7 @@ __global__ void __launch_bounds__(256) k_csr_epi(CsrView A, const XT* __restrict
   for (uint32_t rb = blockIdx.x * gpb; rb < A.rows; rb += stride) {
     const uint32_t row = rb + threadIdx.x / G;
     AT sum = AT(0);
-    if (row < A.rows) sum = csr_row<G, VT, XT, AT>(val, A.col, x, __ldg(A.rp + row), __ldg(A.rp + row + 1), sub);
+    if (row < A.rows) sum = csr_row<G, P, VT, XT, AT>(val, A.col, x, __ldg(A.rp + row), __ldg(A.rp + row + 1), sub);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, G);
     if (sub == 0 && row < A.rows) acc += epi(row, sum);

@@ -8,7 +8,7 @@
 
 namespace fb {
 
-template<typename T, int G, typename IT>
+template<typename T, int G, int P, typename IT>
 __global__ void __launch_bounds__(256) k_csr(T* r, T a, const T* __restrict__ x, T b, const T* y,
                                              const T* __restrict__ val, const IT* __restrict__ col,
                                              const IT* __restrict__ rp, uint64_t rows, bool use_y) {
@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(256) k_csr(T* r, T a, const T* __restrict__ x,
   if (row >= rows) return;  // whole sub-group exits together (G divides 32)
   T prev(0);
   if (use_y && sub == 0) prev = y[row];
-  T sum = csr_row<G, T, T, T>(val, col, x, __ldg(rp + row), __ldg(rp + row + 1), sub);
+  T sum = csr_row<G, P, T, T, T>(val, col, x, __ldg(rp + row), __ldg(rp + row + 1), sub);
   const unsigned mask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o, G);
@@ -116,18 +116,24 @@ int csr_apply(T* r, T a, const T* x, T b, const T* y, const T* val, const IT* co
   //   75 (8), 135 (16); 16 entries, 1.0M rows, FP64 u64: 60 (4), 68 (8), 82 (2); 9 entries, 1.44M rows,
   //   FP64 u32: 45 (2), 49 (4), 84 (8); 3.4 entries, 2.1M rows, FP32 u32: 17 (1), 33 (2), 51 (4)
   // One entry at a time with 8 threads per row (2 for the last) took 117, 103, 109, 94, 98 and 39 us.
+  // The sums per thread (P, csr_row) go by the rounding. FP32 errors against 64 bits over the groups P G, in
+  // units of 1e-8: 3D prolongation 2.86 (1), 2.75 (2), 2.74 (4); random rows of 6 entries 4.48 (2), 4.80
+  // (4); 2D stencil, 9 entries, 5.03 (2), 5.04 (4), 5.18 (8); 2D restriction, 9, 5.14 (2), 5.03 (4), 4.76
+  // (8); random rows of 16 5.56 (4), 5.62 (8), of 27 6.32 (4), 6.04 (8); 3D restriction, 27, 6.46 (4), 6.00 (8).
   const double avg = rows ? double(nnz) / double(rows) : 0.0;
   constexpr bool wide = sizeof(T) + sizeof(IT) >= 12;
-  auto launch = [&](auto g) {
-    constexpr int G = decltype(g)::value;
-    k_csr<T, G, IT><<<grid_for(rows * G, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
+  auto launch = [&](auto g, auto p) {
+    constexpr int G = decltype(g)::value, P = decltype(p)::value;
+    k_csr<T, G, P, IT><<<grid_for(rows * G, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
   };
-  if (avg <= 4.0) launch(std::integral_constant<int, 1>());
-  else if (avg <= 12.0) launch(std::integral_constant<int, 2>());
-  else if (avg <= 20.0) launch(std::integral_constant<int, 4>());
-  else if (avg <= 32.0) launch(std::integral_constant<int, wide ? 8 : 4>());
-  else if (avg <= 64.0) launch(std::integral_constant<int, wide ? 16 : 8>());
-  else launch(std::integral_constant<int, 32>());
+  using std::integral_constant;
+  if (avg <= 4.0) launch(integral_constant<int, 1>(), integral_constant<int, 2>());
+  else if (avg <= 8.0) launch(integral_constant<int, 2>(), integral_constant<int, 1>());
+  else if (avg <= 12.0) launch(integral_constant<int, 2>(), integral_constant<int, 2>());
+  else if (avg <= 20.0) launch(integral_constant<int, 4>(), integral_constant<int, 1>());
+  else if (avg <= 32.0) launch(integral_constant<int, wide ? 8 : 4>(), integral_constant<int, wide ? 1 : 2>());
+  else if (avg <= 64.0) launch(integral_constant<int, wide ? 16 : 8>(), integral_constant<int, wide ? 1 : 2>());
+  else launch(integral_constant<int, 32>(), integral_constant<int, 1>());
   FB_CHECK_LAUNCH();
   return FB_OK;
 }

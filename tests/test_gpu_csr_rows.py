@@ -41,6 +41,35 @@ def test_rows(name, dtype, eps, index):
     assert np.all(abs(A.apply(R, X, Y, -1.0).numpy() - (y - S @ x)) <= bound)
 
 
+@pytest.mark.parametrize("index", ["u32", "u64"])
+@pytest.mark.parametrize("name", sorted(LENGTHS))
+def test_terms_are_summed_in_groups(name, index):
+    """FP32: however many threads share a row, its terms are summed in 2, 4, 8, 16 or 32 groups (up to
+    8, 20, 32, 64 and more entries a row), each with one running sum, which are then added pairwise"""
+    from feat3_b200.lafem import DenseVector, SparseMatrixCSR
+    rng = np.random.default_rng(4)
+    n, m = 777, 2000
+    rl = LENGTHS[name](rng, n)
+    rp = np.concatenate([[0], np.cumsum(rl)])
+    ci = np.concatenate([np.sort(rng.choice(m, k, replace=False)) for k in rl] + [np.zeros(0, np.int64)]).astype(np.int64)
+    va, x = rng.standard_normal(ci.size).astype(np.float32), rng.standard_normal(m).astype(np.float32)
+    A = SparseMatrixCSR(rp, ci, va, columns=m, dtype=torch.float32, index=index)
+    X, R = DenseVector(torch.tensor(x).cuda()), DenseVector(torch.full((n,), np.nan).cuda())
+    out = A.apply(R, X).numpy()
+    avg = ci.size / n
+    g = 2 if avg <= 8 else 4 if avg <= 20 else 8 if avg <= 32 else 16 if avg <= 64 else 32
+    ref = np.zeros(n, np.float32)
+    for i in range(n):
+        s = np.zeros(g, np.float32)
+        for k in range(rp[i], rp[i + 1]):  # one rounding (fused multiply-add): the FP64 product is exact
+            s[(k - rp[i]) % g] = np.float32(float(va[k]) * float(x[ci[k]]) + float(s[(k - rp[i]) % g]))
+        while s.size > 1:
+            s = s[:s.size // 2] + s[s.size // 2:]
+        ref[i] = s[0]
+    # (the reference rounds twice, to 53 and to 24 bits: another last bit in 1 of 2^29 terms)
+    assert np.count_nonzero(out != ref) <= 1
+
+
 @pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
 @pytest.mark.parametrize("avg", [3, 9, 16, 27, 50, 125])
 def test_last_row_at_the_index_limit(avg, dtype, eps):
