@@ -1061,7 +1061,8 @@ static int launch_dense(fb_mg* m, int l, const T* b) {
 
 // Forms the dense operator of the small end (V-cycle with the fixed coarse-grid correction, a linear
 // coarse solver): the first level below the finest with at most kDenseRows rows, when it is not the
-// coarsest one already.
+// coarsest one already. A second configuration with the same smoother and coarse solver (another
+// tolerance, outer solver or format) keeps it.
 template<typename T, int NC>
 static int launch_dense_build(fb_mg* m, const DenseArgs& D, T* op, size_t smem) {
   auto fn = k_dense_build<T, NC>;
@@ -1073,13 +1074,20 @@ static int launch_dense_build(fb_mg* m, const DenseArgs& D, T* op, size_t smem) 
 }
 
 template<typename T>
-static int build_dense(fb_mg* m, T** op) {
+static int build_dense(fb_mg* m, T** op, DenseKey* key) {
   const int nl = (int)m->L.size();
   m->dense_l = 0;
   if (m->cfg.cycle != FB_CYCLE_V || m->cfg.adapt_cgc != FB_CGC_FIXED || m->cfg.coarse == FB_COARSE_PCG) return FB_OK;
   int ld = 1;
   while (ld < nl && m->L[ld].n > kDenseRows) ++ld;
   if (ld >= nl - 1 || nl - ld > kDenseMax) return FB_OK;
+  DenseKey want;
+  want.nu = m->cfg.nu; want.coarse = m->cfg.coarse;
+  want.omega_jac = m->cfg.omega_jac; want.omega_rich = m->cfg.omega_rich;
+  if (*key == want) {
+    m->dense_l = ld;
+    return FB_OK;
+  }
   DenseArgs D{};
   D.nlv = nl - ld; D.nu = m->cfg.nu; D.coarse = m->cfg.coarse; D.omega = m->cfg.omega_rich;
   D.cinv = m->cinv64; D.ldc = dense_ld(m->L[nl - 1].n);
@@ -1097,9 +1105,11 @@ static int build_dense(fb_mg* m, T** op) {
   const uint32_t n = m->L[ld].n;
   const uint64_t size = uint64_t(n) * dense_ld(n);
   if (!*op && dalloc(m, op, size) != FB_OK) return FB_OK;  // no room: level by level
+  *key = DenseKey();  // (of no use until the launch below has gone out)
   FB_CUDA(cudaMemsetAsync(*op, 0, sizeof(T) * size, m->stream));
   if (2 * per <= cap) FB_TRY((launch_dense_build<T, 2>(m, D, *op, 2 * per)));
   else FB_TRY((launch_dense_build<T, 1>(m, D, *op, per)));
+  *key = want;
   m->dense_l = ld;
   return FB_OK;
 }
@@ -1918,7 +1928,7 @@ static int ensure_vectors(fb_mg* m, int prec) {
     k_cvt<float, double><<<ew_grid(size), 256, 0, m->stream>>>(m->cinv32, m->cinv64, size);
     FB_CHECK_LAUNCH();
   }
-  FB_TRY(low ? build_dense<float>(m, &m->dop32) : build_dense<double>(m, &m->dop64));
+  FB_TRY(low ? build_dense<float>(m, &m->dop32, &m->dkey32) : build_dense<double>(m, &m->dop64, &m->dkey64));
   const uint32_t n = m->L[0].n;
   if (!m->r) {
     FB_TRY(dalloc(m, &m->r, n)); FB_TRY(dalloc(m, &m->p, n)); FB_TRY(dalloc(m, &m->q, n));

@@ -114,6 +114,16 @@ struct Level {
 // structured hierarchy; a no-op for what exists already
 int ensure_assembled(fb_mg* m, bool matrices, bool transfers);
 
+// The part of a configuration that the dense operator depends on (the matrices, transfers and filters of
+// a hierarchy do not change); nu = 0: none formed
+struct DenseKey {
+  int nu = 0, coarse = 0;
+  double omega_jac = 0.0, omega_rich = 0.0;
+  bool operator==(const DenseKey& o) const {
+    return nu == o.nu && coarse == o.coarse && omega_jac == o.omega_jac && omega_rich == o.omega_rich;
+  }
+};
+
 }  // namespace fb
 
 struct fb_mg {
@@ -147,6 +157,7 @@ struct fb_mg {
   bool dense_on = true;
   double* dop64 = nullptr;
   float* dop32 = nullptr;
+  fb::DenseKey dkey64, dkey32;   // what they were formed with
   // outer (finest) vectors
   double *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *xb = nullptr, *bb = nullptr;
   float* p32 = nullptr;          // FP32 search direction of the mixed matrix-free form

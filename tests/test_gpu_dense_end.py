@@ -104,3 +104,25 @@ def test_tiny_and_non_finite_defects(case, fmt):
                     ref = H.vcycle(t, nu=nu, coarse=coarse, inner=prec)
                 np.testing.assert_array_equal(mg.vcycle(torch.tensor(t).cuda()).cpu().numpy(), ref)
     mg.close()
+
+
+def test_operator_follows_the_configuration():
+    """the operator is kept over configurations that do not change it and formed again for those that
+    do, in each element type: every cycle against the oracle's"""
+    from feat3_b200.solver import MultiGrid
+    k = coefficient(2, 6)
+    H = po.Hierarchy(2, 1, 6, 1, k)
+    d = H.rhs("one")
+    mg = MultiGrid.structured(2, 1, 6, 1, k)
+    base = dict(nu=2, omega_jac=0.5, omega_rich=1.0, coarse="direct")
+    runs = [{}, dict(tol=1e-4), dict(nu=3), dict(nu=3, precision="f32"), dict(precision="f32"), {}, dict(omega_jac=0.6),
+            dict(omega_rich=0.9), dict(omega_rich=0.9, outer="richardson"), dict(coarse="none"), dict(cycle="w"),
+            dict(coarse="none"), dict(precision="f16"), dict(precision="f32", omega_jac=0.6), dict(cgc="energy"), {},
+            dict(format="matfree")]
+    for run in runs:
+        mg.configure(**{**base, **run})
+        ref = H.vcycle(d, **{n: v for n, v in {**base, **run}.items() if n in (*base, "cycle", "cgc")})
+        out = mg.vcycle(torch.tensor(d).cuda()).cpu().numpy()
+        # FP16: values of 11 bits on the finest level
+        assert relerr(out, ref) <= {"f64": 1e-13, "f32": 6e-6, "f16": 5e-3}[run.get("precision", "f64")], run
+    mg.close()
