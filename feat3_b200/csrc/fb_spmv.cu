@@ -9,20 +9,15 @@
 namespace fb {
 
 template<typename T, int G, int P, typename IT>
-__global__ void __launch_bounds__(256) k_csr(T* r, T a, const T* __restrict__ x, T b, const T* y,
+__global__ void __launch_bounds__(256, 8) k_csr(T* r, T a, const T* __restrict__ x, T b, const T* y,
                                              const T* __restrict__ val, const IT* __restrict__ col,
                                              const IT* __restrict__ rp, uint64_t rows, bool use_y) {
-  const uint64_t gid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  const uint64_t row = gid / G;
-  const int sub = threadIdx.x % G;
-  if (row >= rows) return;  // whole sub-group exits together (G divides 32)
+  const uint64_t row = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) / G;
+  const bool has = row < rows, first = has && threadIdx.x % G == 0;
   T prev(0);
-  if (use_y && sub == 0) prev = y[row];
-  T sum = csr_row<G, P, T, T, T>(val, col, x, __ldg(rp + row), __ldg(rp + row + 1), sub);
-  const unsigned mask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o, G);
-  if (sub == 0) r[row] = use_y ? (sum * a) + (b * prev) : sum * a;
+  if (use_y && first) prev = y[row];
+  const T sum = csr_rows<G, P, T, T, T>(val, col, x, has ? __ldg(rp + row) : IT(0), has ? __ldg(rp + row + 1) : IT(0));
+  if (first) r[row] = use_y ? (sum * a) + (b * prev) : sum * a;
 }
 
 template<typename T>

@@ -16,6 +16,7 @@ LENGTHS = {
     "27": lambda rng, n: np.full(n, 27),
     "33_to_60": lambda rng, n: rng.integers(33, 61, n),
     "125": lambda rng, n: np.full(n, 125),
+    "long_rows": lambda rng, n: np.where((n - 1 - np.arange(n)) % 13 == 0, rng.integers(30, 36, n), rng.integers(0, 2, n)),
     "one_long": lambda rng, n: np.where(np.arange(n) == n // 2, 1500, rng.integers(0, 4, n)),
 }
 
@@ -58,11 +59,12 @@ def test_terms_are_summed_in_groups(name, index):
     out = A.apply(R, X).numpy()
     avg = ci.size / n
     g = 2 if avg <= 8 else 4 if avg <= 20 else 8 if avg <= 32 else 16 if avg <= 64 else 32
+    threads = 1 if avg <= 4 else 2 if avg <= 12 else 4 if avg <= 20 or (avg <= 32 and index == "u32") else 8
     ref = np.zeros(n, np.float32)
     for i in range(n):
-        s = np.zeros(g, np.float32)
+        s = np.zeros(32 if rl[i] > 32 * threads and avg <= 64 else g, np.float32)  # (a whole warp for a long row)
         for k in range(rp[i], rp[i + 1]):  # one rounding (fused multiply-add): the FP64 product is exact
-            s[(k - rp[i]) % g] = np.float32(float(va[k]) * float(x[ci[k]]) + float(s[(k - rp[i]) % g]))
+            s[(k - rp[i]) % s.size] = np.float32(float(va[k]) * float(x[ci[k]]) + float(s[(k - rp[i]) % s.size]))
         while s.size > 1:
             s = s[:s.size // 2] + s[s.size // 2:]
         ref[i] = s[0]
