@@ -25,7 +25,6 @@ int workspace_get(Workspace** out) {
     Workspace* w = new Workspace();
     if (cudaMalloc(&w->partials, sizeof(double) * kRedBlocks) != cudaSuccess ||
         cudaMalloc(&w->counter, sizeof(unsigned) * 8) != cudaSuccess ||
-        cudaMalloc(&w->result, sizeof(double) * 8) != cudaSuccess ||
         cudaMallocHost(&w->host_result, sizeof(double) * 8) != cudaSuccess) {
       delete w;
       return FB_ERR_ALLOC;

@@ -161,7 +161,8 @@ __device__ __forceinline__ bool reduce_finish_nd(double blk, double* ws, unsigne
 struct Workspace {
   double* partials = nullptr;   // kRedBlocks doubles
   unsigned* counter = nullptr;  // one counter per concurrent reduction slot
-  double* result = nullptr;     // device scalar used by the *_sync host-returning variants
+  // pinned host word that the kernels of the *_sync host-returning variants write themselves; valid
+  // after the synchronisation of their stream
   double* host_result = nullptr;
 };
 int workspace_get(Workspace** ws);
