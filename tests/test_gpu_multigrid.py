@@ -189,13 +189,14 @@ def test_adjoint_gradient_matches_oracle():
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32"])
-@pytest.mark.parametrize("dim,lvl", [(3, 5), (2, 7)])
-def test_matfree_fusions_match_unfused(prec, dim, lvl):
+@pytest.mark.parametrize("dim,lvl,lmin", [(3, 5, 1), (3, 5, 3), (2, 7, 1), (2, 7, 5)])  # (no dense small end from 3 and 5)
+def test_matfree_fusions_match_unfused(prec, dim, lvl, lmin):
     """the fused coarse cycle, the r.z fused into the last smoothing step and the tiled
-    operator kernel against the level-by-level, separate-reduction, simple-kernel path"""
+    operator kernel against the level-by-level, separate-reduction, simple-kernel path (2D from level 1
+    on: the last two alone)"""
     from feat3_b200.solver import MultiGrid
     k = lognormal_k(dim, lvl, 1.0, seed=9)
-    mg = MultiGrid.structured(dim, 1, lvl, 1, k)
+    mg = MultiGrid.structured(dim, 1, lvl, lmin, k)
     b = mg.assemble_rhs("one")
     mg.configure(nu=2, precision=prec, format="matfree")
     fused = mg.solve(b)
@@ -304,18 +305,37 @@ def test_unknown_flags_are_rejected():
     mg.close()
 
 
-@pytest.mark.parametrize("dim,lvl,prec", [(3, 6, "f32"), (2, 9, "f32"), (3, 5, "f64"), (2, 8, "f64")])
-def test_coarse_cluster_matches_level_kernels(dim, lvl, prec):
+# Level 0 of the cycle is the finest. size: the defect's norm, or None for the right-hand side as it is.
+# With a dense small end (two or more levels of at most 1,280 rows) the cluster holds the levels above it
+# in 3D and is not used in 2D; without one it holds every level of at most 5,000 rows: where one level is
+# that small, and for defects of at most 1,024 eps^2, which leave the dense operator aside (down to
+# 27 or 9 rows here). The norms keep some of the levels inside the smoothers' skip test.
+CLUSTER = [(dim, lvl, lmin, prec, size)
+           for dim, lvl, lmin, prec in [(3, 6, 1, "f32"), (3, 5, 1, "f64"), (3, 6, 3, "f32"), (3, 5, 3, "f64"),
+                                        (2, 9, 5, "f32"), (2, 8, 5, "f64"), (2, 9, 1, "f32"), (2, 8, 1, "f64")]
+           for size in (None, 500.0, 5.0) if (dim, lmin, size) != (2, 1, None)]
+
+
+@pytest.mark.parametrize("coarse", ["direct", "smoother", "none"])
+@pytest.mark.parametrize("dim,lvl,lmin,prec,size", CLUSTER)
+def test_coarse_cluster_matches_level_kernels(dim, lvl, lmin, prec, coarse, size):
     """the fused coarse cycle (one cluster, levels up to 5,000 rows) runs each row's arithmetic of
     the level-by-level kernels in the same order, and its reductions feed only the smoothers' skip
-    tests: one V-cycle is bit-identical with the coarse end fused or level by level"""
+    tests: one V-cycle is bit-identical with the coarse end fused or level by level, and the fused
+    form launches fewer kernels"""
     from feat3_b200.solver import MultiGrid
     k = lognormal_k(dim, lvl, 1.0, seed=19)
-    mg = MultiGrid.structured(dim, 1, lvl, 1, k)
+    mg = MultiGrid.structured(dim, 1, lvl, lmin, k)
     d = mg.assemble_rhs("one")
-    a = mg.configure(nu=2, precision=prec, format="matfree").vcycle(d).cpu().numpy()
-    b = mg.configure(nu=2, precision=prec, format="matfree", fuse_coarse=False).vcycle(d).cpu().numpy()
+    if size is not None:
+        d *= size * (2.0 ** -46 if prec == "f32" else 2.0 ** -104) / float(d.norm())
+    common = dict(nu=2, precision=prec, format="matfree", coarse=coarse, max_iter=1)
+    a = mg.configure(**common).vcycle(d).cpu().numpy()
+    assert any(mg.level_forms(l)[2] for l in range(mg.num_levels())) == (lmin == 1)
+    fused = mg.solve(d)["kernel_launches"]
+    b = mg.configure(fuse_coarse=False, **common).vcycle(d).cpu().numpy()
     np.testing.assert_array_equal(a, b)
+    assert fused < mg.solve(d)["kernel_launches"]
     mg.close()
 
 
