@@ -117,6 +117,7 @@ _SIGS = {
     "fb_mg_element_grad": [vp, vp, vp, vp],
     "fb_mg_time_spmv": [vp, i32, i32, i32, i32, C.POINTER(dbl)],
     "fb_mg_test_expire_wait": [vp],
+    "fb_mg_level_forms": [vp, i32, C.POINTER(u64), C.POINTER(u64), C.POINTER(i32)],
     # container file I/O
     "fb_io_csr_read": [C.c_char_p, i32, C.POINTER(CsrHost)],
     "fb_io_csr_write": [C.c_char_p, i32, C.POINTER(CsrHost), i32],

@@ -2412,6 +2412,23 @@ int fb_mg_test_expire_wait(fb_mg* m) {
   return FB_OK;
 }
 
+int fb_mg_level_forms(fb_mg* m, int level, uint64_t* chunks, uint64_t* patterned, int* dense) {
+  if (!m || level < 0 || level >= (int)m->L.size()) return FB_ERR_INVALID;
+  if (!m->configured) return FB_ERR_NOT_READY;
+  FB_CUDA(cudaSetDevice(m->device));
+  const Level& L = m->L[level];
+  if (chunks) *chunks = L.A.nchunks;
+  if (dense) *dense = m->dense_l > 0 && level == m->dense_l ? 1 : 0;
+  if (!patterned) return FB_OK;
+  *patterned = 0;
+  if (!L.A.md || use_matfree(m, L) || use_stencil(m, L)) return FB_OK;
+  std::vector<uint32_t> md(L.A.nchunks);
+  FB_CUDA(cudaMemcpyAsync(md.data(), L.A.md, sizeof(uint32_t) * md.size(), cudaMemcpyDeviceToHost, m->stream));
+  FB_CUDA(cudaStreamSynchronize(m->stream));
+  for (uint32_t v : md) *patterned += (v >> 28) != 0;
+  return FB_OK;
+}
+
 int fb_mg_time_spmv(fb_mg* m, int level, int which, int prec, int reps, double* ms) {
   if (!m || !ms || level < 0 || level >= (int)m->L.size() || reps < 1 || which < 0 || which > 3 || prec < 0 || prec > 2)
     return FB_ERR_INVALID;

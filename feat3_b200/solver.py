@@ -149,6 +149,13 @@ class MultiGrid:
     def nnz(self, level=0):
         return int(_lib.load().fb_mg_nnz(self.h, level))
 
+    def level_forms(self, level=0):
+        """(chunks, chunks that follow an offset pattern, V-cycle ends here in its dense operator) of
+        a level under the current configuration (fb_mg_level_forms)"""
+        chunks, pat, dense = C.c_uint64(0), C.c_uint64(0), C.c_int(0)
+        _lib.call("fb_mg_level_forms", self.h, level, C.byref(chunks), C.byref(pat), C.byref(dense))
+        return int(chunks.value), int(pat.value), bool(dense.value)
+
     def export_csr(self, level=0):
         n, nnz = self.ndofs(level), self.nnz(level)
         rp = np.zeros(n + 1, np.uint64)

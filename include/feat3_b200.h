@@ -358,6 +358,12 @@ FB_API int fb_mg_time_spmv(fb_mg* mg, int level, int which, int precision, int r
  * the tests arms it. */
 FB_API int fb_mg_test_expire_wait(fb_mg* mg);
 
+/* Which storage forms the current configuration found for a level (0 = finest): the chunks of its SELL
+ * matrix, how many of them follow an offset pattern (0 where the level's operator does not run on
+ * the SELL matrix), and whether the V-cycle ends on this level in its dense operator. Any output may be
+ * NULL. FB_ERR_NOT_READY before fb_mg_configure. Synchronous. */
+FB_API int fb_mg_level_forms(fb_mg* mg, int level, uint64_t* chunks, uint64_t* patterned, int* dense);
+
 /* ===================================================================================== */
 /* 3. Container file I/O in FEAT3's formats (host only, no device needed)                */
 /* ===================================================================================== */

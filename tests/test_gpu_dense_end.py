@@ -22,6 +22,14 @@ def coefficient(dim, level):
     return np.exp(np.random.default_rng(5).standard_normal((1 << level) ** dim))
 
 
+def dense_levels(H):
+    """per level, finest first: the operator's level, the first below the finest with at most 1,280 rows"""
+    n = [H.ndofs(l) for l in range(H.level, H.level_min - 1, -1)]
+    at = next(i for i in range(1, len(n)) if n[i] <= 1280)
+    assert at < len(n) - 1
+    return [i == at for i in range(len(n))]
+
+
 @pytest.mark.parametrize("case", CASES, ids=["d%dq%dL%d-%d-nu%d-%s" % c for c in CASES])
 @pytest.mark.parametrize("fmt", ["sell", "stencil", "matfree"])
 def test_cycle_matches_oracle(case, fmt):
@@ -37,6 +45,7 @@ def test_cycle_matches_oracle(case, fmt):
     # FP64 to rounding; FP32 within 100 roundings of 2^-24 (some 50 dependent steps)
     for prec, tol in (("f64", 1e-13), ("f32", 6e-6), ("f64", 1e-13)):
         mg.configure(nu=nu, coarse=coarse, precision=prec, format=fmt)
+        assert [mg.level_forms(l)[2] for l in range(mg.num_levels())] == dense_levels(H), prec
         out = mg.vcycle(dd).cpu().numpy()
         assert relerr(out, ref) <= tol, prec
         if prec == "f64":
@@ -44,6 +53,7 @@ def test_cycle_matches_oracle(case, fmt):
             np.testing.assert_array_equal(out, first)
     # the other cycles do not use the operator; the V-cycle after them does again
     mg.configure(nu=nu, coarse=coarse, format=fmt, cycle="w")
+    assert not any(mg.level_forms(l)[2] for l in range(mg.num_levels()))
     mg.vcycle(dd)
     mg.configure(nu=nu, coarse=coarse, format=fmt)
     np.testing.assert_array_equal(mg.vcycle(dd).cpu().numpy(), first)
@@ -63,7 +73,28 @@ def test_handed_hierarchy_matches_oracle(sigma):
         levels.append(e)
     d = H.rhs("one")
     mg = MultiGrid.from_csr(levels, sell_sigma=sigma).configure(nu=3)
+    assert [mg.level_forms(l)[2] for l in range(mg.num_levels())] == dense_levels(H)
     assert relerr(mg.vcycle(torch.tensor(d).cuda()).cpu().numpy(), H.vcycle(d, nu=3)) <= 1e-13
+    mg.close()
+
+
+@pytest.mark.parametrize("case", CASES, ids=["d%dq%dL%d-%d-nu%d-%s" % c for c in CASES])
+@pytest.mark.parametrize("fmt", ["sell", "stencil"])
+def test_fp16_cycle(case, fmt):
+    """FP16 values above the operator's level, which runs in FP32: against the oracle's cycle on
+    unrounded values. The levels above it differ from it by the values' rounding, 2^-11 of each entry
+    (two smoothings and a defect per level pass it on)."""
+    from feat3_b200.solver import MultiGrid
+    dim, deg, lvl, lmin, nu, coarse = case
+    k = coefficient(dim, lvl)
+    H = po.Hierarchy(dim, deg, lvl, lmin, k)
+    d = H.rhs("one") * np.random.default_rng(6).uniform(0.5, 1.5, H.ndofs())
+    mg = MultiGrid.structured(dim, deg, lvl, lmin, k)
+    mg.configure(nu=nu, coarse=coarse, precision="f16", format=fmt)
+    levels = dense_levels(H)
+    assert [mg.level_forms(l)[2] for l in range(mg.num_levels())] == levels
+    out = mg.vcycle(torch.tensor(d).cuda()).cpu().numpy()
+    assert relerr(out, H.vcycle(d, nu=nu, coarse=coarse)) <= 2.0 ** -11 * 2 * (2 * nu + 1) * levels.index(True)
     mg.close()
 
 

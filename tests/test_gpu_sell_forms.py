@@ -64,6 +64,35 @@ CASES = {
     "partial_chunk": lambda: lattice((4133,)),
 }
 
+PATTERNED = {(n, 1) for n in ("q1_2d_70x67", "q1_3d_33", "q1_3d_17", "q2_2d_65", "bands", "diagonal", "partial_chunk")}
+PATTERNED |= {(n, 256) for n in ("q1_2d_70x67", "bands", "diagonal", "partial_chunk")}
+
+
+def patterned_chunks(rp, ci, sigma):
+    """how many chunks follow one of the four patterns kept: the offsets of a full row that every other
+    row of the chunk follows with gaps, whose columns exist for all 32 slot rows; the patterns are the
+    first four met from 256 chunks before the middle on, within 512"""
+    n = rp.size - 1
+    rl = np.diff(rp)
+    perm = np.concatenate([w + np.argsort(-rl[w:w + sigma], kind="stable") for w in range(0, n, sigma)])
+    offsets = []
+    for c in range((n + 31) // 32 if n > 1280 else 0):
+        rows = perm[32 * c:32 * c + 32]
+        lanes = [ci[rp[r]:rp[r + 1]] - (32 * c + t) for t, r in enumerate(rows)]
+        ref = max(lanes, key=len)  # (the first of the longest)
+        at = 32 * c + np.arange(32)[:, None] + ref[None, :]
+        ok = 0 < ref.size <= 32 and at.min() >= 0 and at.max() < n
+        for off in lanes:
+            it = iter(ref)
+            ok = ok and all(any(o == p for p in it) for o in off)
+        offsets.append(tuple(ref) if ok else None)
+    first = max(0, (len(offsets) - 512) // 2)
+    kept = []
+    for off in offsets[first:first + 512]:
+        if off is not None and off not in kept:
+            kept.append(off)
+    return sum(off in kept[:4] for off in offsets if off is not None)
+
 
 @pytest.mark.parametrize("sigma", [1, 256])
 @pytest.mark.parametrize("name", sorted(CASES))
@@ -84,6 +113,9 @@ def test_products(name, sigma):
     mg = MultiGrid.from_csr([{"A": (rp, ci, va), "filter": filt}], sell_sigma=sigma)
     # one Richardson step with the identity preconditioner: x + filter(b - A x)
     mg.configure(outer="richardson", coarse="none", max_iter=1, tol=0.0)
+    expected = patterned_chunks(rp, ci, sigma)
+    assert mg.level_forms(0) == ((n + 31) // 32, expected, False)
+    assert (expected > 0) == ((name, sigma) in PATTERNED)
     u = mg.solve(torch.tensor(b).cuda(), torch.tensor(x).cuda())["u"].cpu().numpy()
     bound = (np.diff(rp) + 3) * EPS["f64"] * (absA @ abs(x) + abs(b) + abs(x))
     assert np.all(abs(u - (x + keep * (b - A @ x))) <= bound)
