@@ -445,6 +445,9 @@ static int build_kron(fb_mg* m, DevCsr& D, int dim, uint32_t rows1, uint32_t col
   D.rows = uint32_t(nrows);
   D.cols = uint32_t(uint64_t(cols1) * cols1 * (dim == 3 ? cols1 : 1));
   D.nnz = nnz;
+  uint32_t longest = 0;
+  for (size_t i = 0; i + 1 < rp.size(); ++i) longest = std::max(longest, rp[i + 1] - rp[i]);
+  D.longest = longest * longest * (dim == 3 ? longest : 1u);
   FB_TRY(dalloc(m, &D.rp, nrows + 1));
   FB_TRY(dalloc(m, &D.col, nnz));
   FB_TRY(dalloc(m, &D.v64, nnz));

@@ -110,7 +110,7 @@ static int launch_csr(fb_mg* m, const DevCsr& A, bool f32, const XT* x, const Ep
   const double avg = A.rows ? double(A.nnz) / double(A.rows) : 0.0;
   auto launch = [&](auto g, auto p) {
     constexpr int G = decltype(g)::value, P = decltype(p)::value;
-    auto fn = k_csr_epi<VT, XT, AT, Epi, G, P>;
+    auto fn = A.longest > 32u * G ? k_csr_epi<VT, XT, AT, Epi, G, P, true> : k_csr_epi<VT, XT, AT, Epi, G, P, false>;
     const int grid = occupancy_grid((const void*)fn, (uint64_t(A.rows) * G + 31) / 32);
     return launch_pdl(m->stream, fn, dim3(grid), dim3(256), 0, A.view(f32), x, epi, m->ws, m->counter, red_out);
   };
@@ -2001,6 +2001,8 @@ int upload_sell(fb_mg* m, DevSell& S, const HostCsr& A, int sigma) {
 int upload_csr(fb_mg* m, DevCsr& D, const HostCsr& A) {
   if (A.rows > 0xffffffffull || A.rp[A.rows] > 0xffffffffull) return FB_ERR_INVALID;
   D.rows = uint32_t(A.rows); D.cols = uint32_t(A.cols); D.nnz = A.rp[A.rows];
+  D.longest = 0;
+  for (uint64_t i = 0; i < A.rows; ++i) D.longest = std::max<uint32_t>(D.longest, uint32_t(A.rp[i + 1] - A.rp[i]));
   std::vector<uint32_t> rp(A.rp.begin(), A.rp.end());
   FB_TRY(dupload(m, &D.rp, rp.data(), rp.size()));
   FB_TRY(dupload(m, &D.col, A.ci.data(), A.ci.size()));

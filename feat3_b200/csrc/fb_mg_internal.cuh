@@ -55,6 +55,7 @@ struct DevSell {
 struct DevCsr {
   uint32_t rows = 0, cols = 0;
   uint64_t nnz = 0;
+  uint32_t longest = 0;     // entries of the longest row
   uint32_t *rp = nullptr, *col = nullptr;
   double* v64 = nullptr;
   float* v32 = nullptr;

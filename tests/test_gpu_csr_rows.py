@@ -103,3 +103,43 @@ def test_last_row_at_the_index_limit(avg, dtype, eps):
         _lib.call("fb_csr_apply_" + sfx, R.data_ptr(), 1.0, X.data_ptr(), 0.0, None, *args, n, m, avg * n, 1, st)
         bound = (n + 3) * eps * (abs(S).T @ abs(x[:n]))
         assert np.all(abs(R.double().cpu().numpy() - S.T @ x[:n]) <= bound)
+
+
+@pytest.mark.parametrize("prec,eps", [("f64", 2.0 ** -53), ("f32", 2.0 ** -24)])
+@pytest.mark.parametrize("long_p,long_r", [(0, 0), (33, 0), (200, 0), (0, 300), (200, 300)])
+def test_transfers_with_long_rows(long_p, long_r, prec, eps):
+    """one cycle on two handed-over levels whose prolongation or restriction has a row that is much
+    longer than the mean, against the same in NumPy"""
+    from feat3_b200.solver import MultiGrid
+    rng = np.random.default_rng(8)
+    n, nc = 3000, 700
+    def diagonal_plus(m):
+        B = sp.random(m, m, 4.0 / m, random_state=rng, format="csr")
+        A = sp.csr_matrix(B + B.T + 8.0 * sp.identity(m))
+        A.sort_indices()
+        return A
+    def transfer(rows, cols, k, row, length):
+        T = sp.lil_matrix(sp.random(rows, cols, k / cols, random_state=rng))
+        if length:
+            T[row, np.sort(rng.choice(cols, length, replace=False))] = rng.uniform(0.1, 1.0, length)
+        T = sp.csr_matrix(T)
+        T.sort_indices()
+        return T
+    A, Ac = diagonal_plus(n), diagonal_plus(nc)
+    P, R = transfer(n, nc, 2.0, n - 1, long_p), transfer(nc, n, 9.0, 17, long_r)
+    csr = lambda M: (M.indptr, M.indices, M.data)
+    none = np.zeros(0, np.int64)
+    mg = MultiGrid.from_csr([{"A": csr(A), "P": csr(P), "R": csr(R), "filter": none}, {"A": csr(Ac), "filter": none}])
+    mg.configure(nu=1, coarse="none", precision=prec)
+    b = rng.standard_normal(n)
+    w = 0.5 / A.diagonal()
+    s = w * b
+    c = R @ (b - A @ s)
+    x = s + P @ c
+    z = mg.vcycle(torch.tensor(b).cuda()).cpu().numpy()
+    # roundings of every term on its way, as many as the longest rows have entries
+    terms = lambda M: abs(M)
+    at = abs(w * b) + terms(P) @ (terms(R) @ (abs(b) + terms(A) @ abs(s)))
+    at = at + abs(w) * (abs(b) + terms(A) @ at)
+    assert np.all(abs(z - (x + w * (b - A @ x))) <= (long_p + long_r + 40) * eps * at)
+    mg.close()
