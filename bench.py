@@ -437,7 +437,7 @@ def native_arm(args):
                                   "storage": "FP16 stencil values (SELL-32, implicit columns) + matrix-free transfers"},
             "fp64": {"time_s": t_fp64, "iters": it64[-1], "dof_it_per_s": n * it64[-1] / t_fp64,
                      "final_rel_residual": r64["hist"][-1] / r64["hist"][0],
-                     "storage": "SELL-C-sigma (C=32, 32-bit column indices) + CSR transfers (drop-in form)"},
+                     "storage": "SELL-C-sigma (C=32, offset patterns, else 32-bit column indices) + CSR transfers (drop-in form)"},
             "fp64_stencil": {"time_s": t_fp64s, "iters": it64s[-1], "dof_it_per_s": n * it64s[-1] / t_fp64s,
                              "storage": "SELL-32 with implicit stencil columns + matrix-free Q1 transfers"},
             "fp64_matfree": {"time_s": t_fp64m, "iters": it64m[-1], "dof_it_per_s": n * it64m[-1] / t_fp64m,

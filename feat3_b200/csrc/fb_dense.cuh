@@ -7,10 +7,11 @@
 // forms it column by column in FP64 when the solver is configured; a cycle then applies it as one
 // matrix-vector product (dense_rows) in place of some 2 nu + 3 dependent launches per level, each of
 // which costs its latency (2-4 us) for a few KB of work.
-// Whole solves with / without it: 2D Q1 129^2 FP64 V(4,4) 0.65 / 1.19 ms, 65^3 FP64 handed over as CSR
-// 3.55 / 4.29 ms, 2D Q2 1025^2 on FP16 values 19.2 / 22.3 ms, 257^3 mixed matrix-free 14.13 / 14.40 ms
-// (its coarse cluster then runs one level instead of four); it adds 0.3-0.4 ms to the configuration. In the
-// FP32 and FP16 forms these levels' matrices enter in FP64 and only the operator is rounded.
+// Whole solves with / without it: 2D Q1 129^2 FP64 V(4,4) 0.53 / 0.96 ms, 65^3 FP64 handed over as CSR
+// 2.82 / 3.33 ms, 2D Q2 1025^2 on FP16 values 12.0 / 14.0 ms, 513^2 solve and adjoint 4.78 / 6.56 ms, 257^3
+// mixed matrix-free 13.26 / 13.84 ms (its coarse cluster then runs one level instead of four); 129^3 FP32
+// cycle 0.487 / 0.533 ms. It adds 0.1 to 0.6 ms to a hierarchy's first configuration. In the FP32 and FP16
+// forms these levels' matrices enter in FP64 and only the operator is rounded.
 #pragma once
 #include "fb_sell.cuh"
 

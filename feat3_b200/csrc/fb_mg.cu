@@ -55,7 +55,9 @@ static int occupancy_grid(const void* fn, uint64_t work_warps) {
 // and its launch latency, which such a kernel mostly consists of, overlaps it. Limits of 0 / 150 /
 // 300 / 800 CTAs / none, in us: 2D Q1 129^2 FP64 solve 578 / 528 / 528 / 529 / 527, 65^3 FP64 handed
 // 2832 / 2767 / 2801 / 2750 / 2840, 1025^2 Q2 FP16 13460 / 13120 / 13005 / 13070 / 13055, 129^3 FP32
-// cycle 526 / 504 / 500 / 500 / 475, 257^3 mixed 14350 / 14290 / 14140 / 14150 / 14820.
+// cycle 526 / 504 / 500 / 500 / 475, 257^3 mixed 14350 / 14290 / 14140 / 14150 / 14820. The mixed solve
+// sets the limit: its large grids lose with the attribute (its figures from 0 to 800 CTAs lie within what
+// runs on different boxes differ), while the SELL and CSR kernels of the FP32 cycle gain at any size.
 constexpr uint64_t kPdlCtas = 300;
 template<typename... KArgs, typename... Args>
 static cudaError_t launch_pdl(cudaStream_t s, void (*fn)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
@@ -1036,7 +1038,8 @@ static int last_solver(const fb_mg* m) { return dense_level(m) > 0 ? FB_COARSE_D
 // smooth were typically above 1e-3 d (the smallest on 25 rows). So above 1024 eps^2 the test would not
 // act, or only on parts a thousand times smaller than the cycle; the upper bounds keep every sum of
 // squares finite. All other cycles run level by level, with the tests. Tiny defects are met at the end of
-// FP32 solves: the 257^3 mixed solve runs its last two iterations level by level, 13.71 -> 13.77 ms.
+// FP32 solves: the 257^3 mixed solve runs its last one or two iterations level by level, 13.71 -> 13.77
+// ms.
 static bool dense_applies(const fb_mg* m, double d) {
   if (m->dense_l == 0) return true;
   const bool low = m->cfg.precision != FB_PREC_F64;

@@ -88,8 +88,8 @@ __device__ __forceinline__ bool smoother_skip(const double* sumsq) {
 // level's scalar without waiting for the result. The ordered finish (reduce_finish: a memory fence, a
 // counter and the last block's second pass) cost each of these launches about 2 us of latency: 2D Q1
 // 129^2 FP64 solve 483 against 527 us, 513^2 solve and adjoint 4.80 against 5.63 ms, 129^3 mixed
-// matrix-free solve 3.19 against 3.41 ms, 257^3 13.86 against 14.13 ms. The other sums, which enter the iterates or are returned, keep it. The scalar starts from zero: the
-// restriction from a level clears that level's defect norm (`clear`), whose readers are done, and the
+// matrix-free solve 3.19 against 3.41 ms. The other sums, which enter the iterates or are returned, keep
+// it. The scalar starts from zero: the restriction from a level clears that level's defect norm (`clear`), whose readers are done, and the
 // first post-smoothing step of a level clears the next coarser level's right-hand-side norm.
 template<typename Epi, typename = void> struct IsNorm { static constexpr bool value = false; };
 template<typename Epi> struct IsNorm<Epi, typename std::enable_if<Epi::kNorm>::type> { static constexpr bool value = true; };
