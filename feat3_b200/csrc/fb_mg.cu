@@ -1675,8 +1675,8 @@ static int run_body(fb_mg* m, int j) {
 // with an entry in every slot (the reference lane) sets the offsets, and every other row's entries
 // follow them in the same order, with gaps (a lattice row next to the boundary, a Q2 edge row
 // between vertex rows). The row's entries move to the slots they match and the gaps hold value -0.0
-// (column ~0u in the 32-bit array, the mark of an empty slot); a chunk with gaps and an entry of -0.0
-// stays plain. Every slot row + offset is a valid column for all 32 lanes. The products and their order
+// (column ~0u in the 32-bit array, the mark of an empty slot); a chunk with an entry of -0.0 stays
+// plain. Every slot row + offset is a valid column for all 32 lanes. The products and their order
 // are those of the plain form.
 struct SellSetup {
   uint32_t rows, cols, nchunks;
@@ -1704,10 +1704,6 @@ __global__ void __launch_bounds__(256) k_sell_candidates(SellSetup S) {
       ok = __all_sync(0xffffffffu, mine >= 0 && mine < int64_t(S.cols));
     }
     ok = __all_sync(0xffffffffu, ok && k == mylen);
-    if (ok && __any_sync(0xffffffffu, mylen < len)) {
-      for (k = 0; k < mylen; ++k) ok = ok && !sell_gap(S.val[e0 + k * 32u + lane]);
-      ok = __all_sync(0xffffffffu, ok);
-    }
     if (lane == 0) S.md[c] = ok ? len | uint32_t(ref + 1) << 23 : 0u;
   }
 }
@@ -1770,11 +1766,16 @@ __global__ void __launch_bounds__(256) k_sell_forms(SellSetup S) {
         if (sell_follows(S, S.pat + p * kSellPatternSlots, S.plen[p], off, len, lane)) form = p + 1;
     }
     const uint32_t mylen = sr < S.rows ? S.rl[S.perm ? S.perm[sr] : sr] : 0u;
+    uint32_t* cp = S.col + e0 + lane;
+    double* vp = S.val + e0 + lane;
+    if (form) {
+      bool ok = true;  // an entry of -0.0 would be taken for an empty slot
+      for (uint32_t j = 0; j < mylen; ++j) ok = ok && !sell_gap(vp[j * 32u]);
+      if (!__all_sync(0xffffffffu, ok)) form = 0;
+    }
     __syncwarp();
     if (lane == 0) S.md[c] = len | (form << 28);
     if (!form) continue;
-    uint32_t* cp = S.col + e0 + lane;
-    double* vp = S.val + e0 + lane;
     uint32_t k = mylen;  // from the last slot down: an entry only moves to a slot at or behind its own
     for (uint32_t j = len; j-- > 0;) {
       const uint32_t at = sr + uint32_t(S.pat[(form - 1) * kSellPatternSlots + j]);
