@@ -516,14 +516,14 @@ __device__ __noinline__ AT csr_long_rows(const VT* val, const IT* col, const XT*
 
 // The product of the row [beg, end) that G lanes share, for all rows of a warp at once (all 32 lanes
 // call it; beg = end where there is no row); valid in the group's first lane. G goes by the mean row
-// length, so rows that are much longer (a constraint that couples everything) are summed by the whole
-// warp: 1.0M rows of 3 entries with 1000 rows of 1000, FP64 u32, 25 us; 115 with one thread for them, 89
+// length, so for up to four threads a row rows that are much longer (a constraint that couples everything)
+// are summed by the whole warp: 1.0M rows of 3 entries with 1000 rows of 1000, FP64 u32, 25 us; 115 with one thread for them, 89
 // with two and one entry loaded at a time. The kernels stay within 32 registers (8 CTAs per SM): 27
 // entries a row, FP64 u64, 81 us, with the compiler's choice of 40 registers 107.
 template<int G, int P, typename VT, typename XT, typename AT, typename IT>
 __device__ __forceinline__ AT csr_rows(const VT* __restrict__ val, const IT* __restrict__ col, const XT* __restrict__ x,
                                        IT beg, IT end) {
-  if constexpr (G < 32)
+  if constexpr (G < 8)
     if (__any_sync(0xffffffffu, end - beg > IT(32 * G))) return csr_long_rows<G, P, VT, XT, AT, IT>(val, col, x, beg, end);
   return group_sum<G>(csr_row<G, P, VT, XT, AT>(val, col, x, beg, end, int(threadIdx.x % G)));
 }

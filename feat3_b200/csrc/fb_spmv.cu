@@ -8,8 +8,9 @@
 
 namespace fb {
 
+// (within 32 registers, 40 for FP32 values with 64-bit indices: 250,000 rows of 27 at random 32 us, 35 with 32)
 template<typename T, int G, int P, typename IT>
-__global__ void __launch_bounds__(256, 8) k_csr(T* r, T a, const T* __restrict__ x, T b, const T* y,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && sizeof(IT) == 8 ? 6 : 8) k_csr(T* r, T a, const T* __restrict__ x, T b, const T* y,
                                              const T* __restrict__ val, const IT* __restrict__ col,
                                              const IT* __restrict__ rp, uint64_t rows, bool use_y) {
   const uint64_t row = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) / G;
@@ -121,14 +122,34 @@ int csr_apply(T* r, T a, const T* x, T b, const T* y, const T* val, const IT* co
     constexpr int G = decltype(g)::value, P = decltype(p)::value;
     k_csr<T, G, P, IT><<<grid_for(rows * G, 256), 256, 0, s>>>(r, a, x, b, y, val, col, rp, rows, use_y);
   };
+  // Few rows: threads enough that most rows are one batch of loads, as long as the matrix is at most some
+  // three fillings of the chip with them (one for rows of up to 4 entries). us with / without: 10,000 rows
+  // of 7 to 11 entries at random, FP64 u32, 2.13 / 2.89, 2D stencil of 401^2 rows 5.2 / 5.5, 1201^2 (not
+  // taken) 45 / 42; 2D Q2 121^2 2.3 / 2.9, 401^2 (not taken) 8.9 / 8.3; 27 entries, FP32 u32, 33^3
+  // 3.1 / 3.2, 51^3 6.5 / 6.4; 3D prolongation, FP64 u32, 33^3 2.05 / 2.45, 65^3 (not taken) 4.7 / 4.3.
   using std::integral_constant;
-  if (avg <= 4.0) launch(integral_constant<int, 1>(), integral_constant<int, 2>());
-  else if (avg <= 8.0) launch(integral_constant<int, 2>(), integral_constant<int, 1>());
-  else if (avg <= 12.0) launch(integral_constant<int, 2>(), integral_constant<int, 2>());
-  else if (avg <= 20.0) launch(integral_constant<int, 4>(), integral_constant<int, 1>());
-  else if (avg <= 32.0) launch(integral_constant<int, wide ? 8 : 4>(), integral_constant<int, wide ? 1 : 2>());
-  else if (avg <= 64.0) launch(integral_constant<int, wide ? 16 : 8>(), integral_constant<int, wide ? 1 : 2>());
-  else launch(integral_constant<int, 32>(), integral_constant<int, 1>());
+  auto few = [&](uint64_t g) { return rows * g <= (uint64_t(1) << 20); };
+  if (avg <= 4.0) {
+    if (rows * 2 <= uint64_t(kSMs) * 2048) launch(integral_constant<int, 2>(), integral_constant<int, 1>());
+    else launch(integral_constant<int, 1>(), integral_constant<int, 2>());
+  } else if (avg <= 8.0) {
+    if (avg > 6.0 && few(4)) launch(integral_constant<int, 4>(), integral_constant<int, 1>());
+    else launch(integral_constant<int, 2>(), integral_constant<int, 1>());
+  } else if (avg <= 12.0) {
+    if (few(4)) launch(integral_constant<int, 4>(), integral_constant<int, 1>());
+    else launch(integral_constant<int, 2>(), integral_constant<int, 2>());
+  } else if (avg <= 20.0) {
+    if (few(8)) launch(integral_constant<int, 8>(), integral_constant<int, 1>());
+    else launch(integral_constant<int, 4>(), integral_constant<int, 1>());
+  } else if (avg <= 32.0) {
+    if (wide || few(8)) launch(integral_constant<int, 8>(), integral_constant<int, 1>());
+    else launch(integral_constant<int, 4>(), integral_constant<int, 2>());
+  } else if (avg <= 64.0) {
+    if (wide || few(16)) launch(integral_constant<int, 16>(), integral_constant<int, 1>());
+    else launch(integral_constant<int, 8>(), integral_constant<int, 2>());
+  } else {
+    launch(integral_constant<int, 32>(), integral_constant<int, 1>());
+  }
   FB_CHECK_LAUNCH();
   return FB_OK;
 }

@@ -16,7 +16,8 @@ LENGTHS = {
     "27": lambda rng, n: np.full(n, 27),
     "33_to_60": lambda rng, n: rng.integers(33, 61, n),
     "125": lambda rng, n: np.full(n, 125),
-    "long_rows": lambda rng, n: np.where((n - 1 - np.arange(n)) % 13 == 0, rng.integers(30, 36, n), rng.integers(0, 2, n)),
+    "4_to_7": lambda rng, n: rng.integers(4, 8, n),
+    "long_rows": lambda rng, n: np.where((n - 1 - np.arange(n)) % 26 == 0, rng.integers(60, 69, n), rng.integers(0, 2, n)),
     "one_long": lambda rng, n: np.where(np.arange(n) == n // 2, 1500, rng.integers(0, 4, n)),
 }
 
@@ -45,8 +46,9 @@ def test_rows(name, dtype, eps, index):
 @pytest.mark.parametrize("index", ["u32", "u64"])
 @pytest.mark.parametrize("name", sorted(LENGTHS))
 def test_terms_are_summed_in_groups(name, index):
-    """FP32: however many threads share a row, its terms are summed in 2, 4, 8, 16 or 32 groups (up to
-    8, 20, 32, 64 and more entries a row), each with one running sum, which are then added pairwise"""
+    """FP32: the terms of a row are summed in 2, 4, 8, 16 or 32 groups (up to 6, 12, 32, 64 and more entries
+    a row), each with one running sum, which are then added pairwise; a row of more than 32 entries per
+    thread (up to four threads) in 32"""
     from feat3_b200.lafem import DenseVector, SparseMatrixCSR
     rng = np.random.default_rng(4)
     n, m = 777, 2000
@@ -58,11 +60,10 @@ def test_terms_are_summed_in_groups(name, index):
     X, R = DenseVector(torch.tensor(x).cuda()), DenseVector(torch.full((n,), np.nan).cuda())
     out = A.apply(R, X).numpy()
     avg = ci.size / n
-    g = 2 if avg <= 8 else 4 if avg <= 20 else 8 if avg <= 32 else 16 if avg <= 64 else 32
-    threads = 1 if avg <= 4 else 2 if avg <= 12 else 4 if avg <= 20 or (avg <= 32 and index == "u32") else 8
+    g = 2 if avg <= 6 else 4 if avg <= 12 else 8 if avg <= 32 else 16 if avg <= 64 else 32
     ref = np.zeros(n, np.float32)
     for i in range(n):
-        s = np.zeros(32 if rl[i] > 32 * threads and avg <= 64 else g, np.float32)  # (a whole warp for a long row)
+        s = np.zeros(32 if rl[i] > 32 * g and g < 8 else g, np.float32)
         for k in range(rp[i], rp[i + 1]):  # one rounding (fused multiply-add): the FP64 product is exact
             s[(k - rp[i]) % s.size] = np.float32(float(va[k]) * float(x[ci[k]]) + float(s[(k - rp[i]) % s.size]))
         while s.size > 1:
@@ -72,26 +73,71 @@ def test_terms_are_summed_in_groups(name, index):
     assert np.count_nonzero(out != ref) <= 1
 
 
+@pytest.mark.parametrize("index", ["u32", "u64"])
+@pytest.mark.parametrize("length,rows,groups", [(3, 160000, 2), (6, 70000, 2), (9, 270000, 4), (16, 135000, 4), (27, 135000, 8),
+                                                (40, 66000, 16)])
+def test_many_rows(length, rows, groups, index):
+    """row counts above which a row gets fewer threads (and several sums in each): the same groups,
+    to the last bit in FP32 as above"""
+    from feat3_b200.lafem import DenseVector, SparseMatrixCSR
+    rng = np.random.default_rng(length)
+    ci = rng.integers(0, rows, (rows, length))
+    va = rng.standard_normal((rows, length)).astype(np.float32)
+    x = rng.standard_normal(rows).astype(np.float32)
+    A = SparseMatrixCSR(np.arange(rows + 1) * length, ci.ravel(), va.ravel(), columns=rows, dtype=torch.float32, index=index)
+    X, R = DenseVector(torch.tensor(x).cuda()), DenseVector(torch.full((rows,), np.nan).cuda())
+    s = np.zeros((rows, groups), np.float32)
+    for j in range(length):
+        t = va[:, j].astype(np.float64) * x[ci[:, j]] + s[:, j % groups]
+        s[:, j % groups] = t.astype(np.float32)
+    while s.shape[1] > 1:
+        s = s[:, :s.shape[1] // 2] + s[:, s.shape[1] // 2:]
+    assert np.count_nonzero(A.apply(R, X).numpy() != s[:, 0]) <= 1
+
+
+@pytest.mark.parametrize("index", ["u32", "u64"])
 @pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
-@pytest.mark.parametrize("avg", [3, 9, 16, 27, 50, 125])
-def test_last_row_at_the_index_limit(avg, dtype, eps):
+def test_many_short_rows_and_long_ones(dtype, eps, index):
+    """one thread per row: rows around its limit of 32 entries and far above it"""
+    from feat3_b200.lafem import DenseVector, SparseMatrixCSR
+    rng = np.random.default_rng(2)
+    n = 170000
+    rl = rng.integers(0, 4, n)
+    rl[rng.choice(n, 3000, replace=False)] = rng.integers(30, 36, 3000)
+    rl[[5, 6, 7, n - 1]] = [3000, 32, 33, 700]
+    rp = np.concatenate([[0], np.cumsum(rl)])
+    ci = rng.integers(0, n, rp[-1])
+    cast = (lambda a: a.astype(np.float32).astype(np.float64)) if dtype == torch.float32 else (lambda a: a)
+    va, x = cast(rng.standard_normal(ci.size)), cast(rng.standard_normal(n))
+    A = SparseMatrixCSR(rp, ci, va, columns=n, dtype=dtype, index=index)
+    X, R = DenseVector(torch.tensor(x, dtype=dtype).cuda()), DenseVector(torch.full((n,), np.nan, dtype=dtype).cuda())
+    S = sp.csr_matrix((va, ci, rp), shape=(n, n), copy=True)
+    bound = (rl + 3) * eps * (sp.csr_matrix((abs(va), ci, rp), shape=(n, n)) @ abs(x))
+    assert np.all(abs(A.apply(R, X).numpy() - S @ x) <= bound)
+
+
+@pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
+@pytest.mark.parametrize("avg,empty", [(3, 0), (7, 0), (9, 0), (27, 0), (50, 0), (125, 0), (3, 200000), (9, 300000),
+                                       (16, 200000), (27, 200000)])
+def test_last_row_at_the_index_limit(avg, empty, dtype, eps):
     """32-bit row pointers up to 2^32 - 1: a lane's next position would lie behind the limit. The
-    arrays start where the first of these rows does (their addresses are shifted by its position), and
-    the mean row length given picks the threads per row."""
+    arrays start where the first of these rows does (their addresses are shifted by its position); the
+    mean row length given and the number of (empty) rows before them pick the threads per row."""
     from feat3_b200 import _lib
     sfx = "f64" if dtype == torch.float64 else "f32"
     rng = np.random.default_rng(avg)
     m = 300
     for rl in ([1, 2, 0, 5], [40, 127, 0, 130], [300, 1], [7]):
         end = 2 ** 32 - 1
+        ci = np.concatenate([np.sort(rng.choice(m, k, replace=False)) for k in rl])
+        rl = [0] * empty + rl
         rp = end - sum(rl) + np.concatenate([[0], np.cumsum(rl)])
         nnz, n = sum(rl), len(rl)
-        ci = np.concatenate([np.sort(rng.choice(m, k, replace=False)) for k in rl])
         va = rng.standard_normal(nnz).astype(np.float32).astype(np.float64)
         x = rng.standard_normal(max(m, n)).astype(np.float32).astype(np.float64)
         S = sp.csr_matrix((va, ci, rp - rp[0]), shape=(n, m), copy=True)
         dev = lambda a, t: torch.tensor(a, dtype=t).cuda()
-        V, X, Y, R = dev(va, dtype), dev(x, dtype), dev(np.zeros(m), dtype), dev(np.full(m, np.nan), dtype)
+        V, X, Y, R = dev(va, dtype), dev(x, dtype), dev(np.zeros(m), dtype), dev(np.full(max(m, n), np.nan), dtype)
         C = torch.tensor(ci.astype(np.uint32).view(np.int32)).cuda()
         P = torch.tensor(rp.astype(np.uint32).view(np.int32)).cuda()
         first = int(rp[0])
@@ -102,7 +148,7 @@ def test_last_row_at_the_index_limit(avg, dtype, eps):
         assert np.all(abs(R[:n].double().cpu().numpy() - S @ x[:m]) <= bound)
         _lib.call("fb_csr_apply_" + sfx, R.data_ptr(), 1.0, X.data_ptr(), 0.0, None, *args, n, m, avg * n, 1, st)
         bound = (n + 3) * eps * (abs(S).T @ abs(x[:n]))
-        assert np.all(abs(R.double().cpu().numpy() - S.T @ x[:n]) <= bound)
+        assert np.all(abs(R[:m].double().cpu().numpy() - S.T @ x[:n]) <= bound)
 
 
 @pytest.mark.parametrize("prec,eps", [("f64", 2.0 ** -53), ("f32", 2.0 ** -24)])
