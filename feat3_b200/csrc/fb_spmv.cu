@@ -45,44 +45,43 @@ __global__ void k_csr_t(T* r, T a, const T* __restrict__ x, const T* __restrict_
 }
 
 // FEAT's SELL-C rows, one thread per row; the loads of eight slots are issued together (two memory
-// round trips per eight slots), and the chunk of a row is found in 32 bits (rows < 2^32), by a shift
-// when C is a power of two (log2C >= 0). 251,000 rows of 9 to 25 FP64 entries, C = 8, 64-bit index:
-// 17.9 -> 16.3 us; matrices of 30,000 rows and less stay at their launch latency (6.2 to 8.2 us).
+// round trips per eight slots). Times over 300 to 400,000 rows of 3 / 9 / 27 entries, C = 8 and 32, against
+// one slot at a time: FP32 u32 1.00 / 0.99 / 1.00, FP32 u64 1.00 / 0.89 / 0.77, FP64 u32 0.97 / 0.95 / 0.95,
+// FP64 u64 1.02 / 1.02 / 0.85. (The row's chunk found by a 32-bit division or a shift: 1.00 / 0.97 / 1.02, 1.15
+// / 1.06 / 0.95, 1.01 / 1.03 / 1.17, 0.96 / 0.97 / 0.94.)
 template<typename T, typename IT>
 __global__ void __launch_bounds__(256) k_ell(T* r, T a, const T* __restrict__ x, T b, const T* y,
                                              const T* __restrict__ val, const IT* __restrict__ col,
                                              const IT* __restrict__ cs, const IT* __restrict__ cl,
-                                             uint32_t C, int log2C, uint32_t rows, bool use_y) {
-  constexpr uint32_t U = 8;
-  const uint64_t at = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (at >= rows) return;
-  const uint32_t row = uint32_t(at);
-  const uint32_t c = log2C >= 0 ? row >> log2C : row / C;
-  const IT base = __ldg(cs + c) + IT(row - c * C);
-  const uint32_t len = uint32_t(__ldg(cl + c));
-  T prev(0);
-  if (use_y) prev = y[row];
+                                             uint32_t C, uint32_t rows, bool use_y) {
+  constexpr int U = 8;
+  const uint64_t row = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  if (row >= rows) return;
+  const uint64_t c = row / C;
+  const IT lane = IT(row % C);
+  const IT base = cs[c] + lane, len = cl[c];
   T sum(0);
-  uint32_t j = 0;
+  IT j = 0;
   for (; j + U <= len; j += U) {
     IT cc[U];
     T vv[U], xx[U];
 #pragma unroll
-    for (uint32_t u = 0; u < U; ++u) {
-      const IT k = base + IT(j + u) * IT(C);
-      cc[u] = __ldg(col + k);
-      vv[u] = __ldg(val + k);
+    for (int u = 0; u < U; ++u) {
+      const IT k = base + (j + IT(u)) * IT(C);
+      cc[u] = col[k];
+      vv[u] = val[k];
     }
 #pragma unroll
-    for (uint32_t u = 0; u < U; ++u) xx[u] = __ldg(x + cc[u]);
+    for (int u = 0; u < U; ++u) xx[u] = x[cc[u]];
 #pragma unroll
-    for (uint32_t u = 0; u < U; ++u) sum += vv[u] * xx[u];
+    for (int u = 0; u < U; ++u) sum += vv[u] * xx[u];
   }
 #pragma unroll 4
   for (; j < len; ++j) {
-    const IT k = base + IT(j) * IT(C);
-    sum += __ldg(val + k) * __ldg(x + __ldg(col + k));
+    const IT k = base + j * IT(C);
+    sum += val[k] * x[col[k]];
   }
+  const T prev = use_y ? y[row] : T(0);
   r[row] = use_y ? (sum * a) + (b * prev) : sum * a;
 }
 
@@ -161,10 +160,7 @@ int ell_apply(T* r, T a, const T* x, T b, const T* y, const T* val, const IT* co
   if (rows == 0) return FB_OK;
   if (!r || (use_y && !y) || !val || !col || !cs || !cl || !x || C == 0 || C > 1024 || rows > 0xffffffffull)
     return FB_ERR_INVALID;
-  int log2C = -1;
-  if ((C & (C - 1)) == 0)
-    for (log2C = 0; (uint64_t(1) << log2C) < C;) ++log2C;
-  k_ell<T, IT><<<grid_for(rows, 256), 256, 0, s>>>(r, a, x, b, y, val, col, cs, cl, uint32_t(C), log2C, uint32_t(rows), use_y);
+  k_ell<T, IT><<<grid_for(rows, 256), 256, 0, s>>>(r, a, x, b, y, val, col, cs, cl, uint32_t(C), uint32_t(rows), use_y);
   FB_CHECK_LAUNCH();
   return FB_OK;
 }
