@@ -70,10 +70,13 @@ void debug_report(cudaError_t e, const char* what, const char* file, int line) {
 }
 
 // ------------------------------------------------------------------ elementwise kernels
-// r = f(x, y) element by element: 16-byte accesses, two in flight per thread and vector, where all
-// vectors are 16-byte aligned (VEC), else one value at a time. An element is read before it is
-// written by the same thread, so r may be x or y. Bound by its streams: 16,974,593 FP32 values in
-// 35 us (axpy, three streams) against 48 us with 4-byte accesses; FP64 66 us either way.
+// r = f(x, y) element by element: 16-byte accesses, two in flight per thread and vector (VEC), or one
+// value at a time. An element is read before it is written by the same thread, so r may be x or y.
+// Bound by its streams: while the L2 holds them, one value at a time is faster. axpy in us, 16-byte accesses
+// against one value: FP32, 1.5 / 4 / 6 / 17 million values 3.8 / 5.4 / 7.1 / 31.9 against 3.2 / 5.5 / 7.9 /
+// 45.1, FP64 5.7 / 14.7 / 25.5 / 63.0 against 4.0 / 10.8 / 24.9 / 66.9 (12 million 45.8 against 47.8); scale,
+// one vector less: FP32 3.1 / 4.7 / 5.9 / 23.3 against 3.0 / 5.1 / 7.0 / 38.5, FP64 4.2 / 7.1 / 12.7 / 44.0
+// against 3.6 / 7.5 / 12.7 / 54.5.
 template<typename T, typename F, int NIN, bool VEC>
 __global__ void __launch_bounds__(256) k_ew(T* r, const T* x, const T* y, uint64_t n, F f) {
   constexpr int NV = VEC ? 16 / sizeof(T) : 1, U = VEC ? 2 : 1;
@@ -134,10 +137,12 @@ __global__ void k_filter_def(T* __restrict__ v, const IT* __restrict__ idx, uint
     v[idx[i]] = T(0);
 }
 
-// dot / sum of squares, FP64 accumulation, deterministic finish. 16-byte loads, four of each vector
-// in flight per thread, where both vectors are 16-byte aligned (VEC); one value per load otherwise.
-// The reads bound it: 16,974,593 FP64 values back to back 49 us (dot, 5.5 TB/s) and 27 us (norm), FP32 29
-// and 12 us, against 71, 60, 68 and 27 us with one value per load.
+// dot / sum of squares, FP64 accumulation, deterministic finish. Four loads of each vector in flight per
+// thread, of 16 bytes (VEC) or of one value. dot in us, 16-byte loads against one value: FP64, 1.5 / 4 / 17
+// million values 6.0 / 8.7 / 46.2 against 5.7 / 8.2 / 41.8, FP32 5.9 / 7.4 / 26.2 against 5.2 / 7.1 / 28.2 (6
+// million 8.1 against 8.6); norm: FP64 5.6 / 7.0 / 24.7 against 5.1 / 6.6 / 26.4 (12 million 12.1 against 14.9),
+// FP32 5.2 / 6.0 / 9.6 against 5.0 / 6.3 / 10.9. One value at a time and none in flight: FP64, 17 million, 69
+// (dot) and 57 (norm). So the FP64 dot never takes 16 bytes.
 template<typename T, bool SQUARE, bool SQRT, bool VEC>
 __global__ void __launch_bounds__(kRedThreads) k_dot(const T* __restrict__ x, const T* __restrict__ y, uint64_t n,
                                                      double* ws, unsigned* counter, double* out) {
@@ -182,12 +187,19 @@ inline unsigned ew_grid(uint64_t n) {
   return g > 16u * kSMs ? 16u * kSMs : g;
 }
 
+// wide accesses: all vectors 16-byte aligned and their streams together longer than `mb` MB, from where on
+// they were faster (figures at k_ew and k_dot)
+inline bool wide_accesses(uintptr_t addresses, uint64_t bytes, uint64_t mb) {
+  return (addresses & 15) == 0 && bytes > mb * 1000000u;
+}
+
 template<int NIN, typename T, typename F>
 int elementwise(T* r, const T* x, const T* y, uint64_t n, F f, cudaStream_t s) {
   if (n == 0) return FB_OK;
   if (!r || !x || (NIN > 1 && !y)) return FB_ERR_INVALID;
   const uintptr_t at = reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(x) | (NIN > 1 ? reinterpret_cast<uintptr_t>(y) : 0);
-  if ((at & 15) == 0) k_ew<T, F, NIN, true><<<ew_grid((n * sizeof(T) + 15) / 16), kEW, 0, s>>>(r, x, y, n, f);
+  constexpr uint64_t mb = NIN > 1 ? (sizeof(T) == 4 ? 60 : 150) : (sizeof(T) == 4 ? 28 : 90);
+  if (wide_accesses(at, n * sizeof(T) * (NIN + 1), mb)) k_ew<T, F, NIN, true><<<ew_grid((n * sizeof(T) + 15) / 16), kEW, 0, s>>>(r, x, y, n, f);
   else k_ew<T, F, NIN, false><<<ew_grid(n), kEW, 0, s>>>(r, x, y, n, f);
   FB_CHECK_LAUNCH();
   return FB_OK;
@@ -208,7 +220,9 @@ int reduce(const T* x, const T* y, uint64_t n, double* result, cudaStream_t s) {
   FB_TRY(workspace_get(&ws));
   unsigned g = grid_for(n, kRedThreads);
   if (g > unsigned(kRedBlocks)) g = kRedBlocks;
-  const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  constexpr uint64_t mb = SQUARE ? (sizeof(T) == 4 ? 10 : 80) : 40;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | (SQUARE ? 0 : reinterpret_cast<uintptr_t>(y));
+  const bool vec = (SQUARE || sizeof(T) == 4) && wide_accesses(at, n * sizeof(T) * (SQUARE ? 1 : 2), mb);
   if (vec) k_dot<T, SQUARE, SQRT, true><<<g, kRedThreads, 0, s>>>(x, y, n, ws->partials, ws->counter, result);
   else k_dot<T, SQUARE, SQRT, false><<<g, kRedThreads, 0, s>>>(x, y, n, ws->partials, ws->counter, result);
   FB_CHECK_LAUNCH();

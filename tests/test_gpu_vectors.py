@@ -1,6 +1,7 @@
 """Vector kernels of the operator layer on aligned and unaligned vectors, in place and not, over sizes
-around the 16-byte packs and the grid's step: bitwise against torch for the single-operation kernels,
-within one rounding of the sum for axpy, and the FP64-accumulated dot and norm."""
+around the 16-byte packs, the grid's step and the lengths from which 16-byte accesses are taken:
+bitwise against torch for the single-operation kernels, within one rounding of the sum for axpy, and
+the FP64-accumulated dot and norm."""
 import numpy as np
 import pytest
 import torch
@@ -9,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shift", [0, 1, 3])
-@pytest.mark.parametrize("n", [1, 2, 3, 5, 31, 1023, 4099, 606208 * 2 + 5, 3000001])
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 31, 1023, 4099, 606208 * 2 + 5, 3000001, 5000003, 6250002,
+                               10000001])
 @pytest.mark.parametrize("dtype,eps", [(torch.float64, 2.0 ** -53), (torch.float32, 2.0 ** -24)])
 def test_vectors(dtype, eps, n, shift):
     from feat3_b200.lafem import DenseVector
