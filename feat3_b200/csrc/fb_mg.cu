@@ -1034,17 +1034,21 @@ static int last_solver(const fb_mg* m) { return dense_level(m) > 0 ? FB_COARSE_D
 // Whether a cycle on a defect of norm d (finest level) may use the dense operator. The operator holds
 // no skip test (smoother_skip), and the test is absolute: a level's smoother is left out where its
 // right-hand side or defect is at most eps^2 (1.4e-14 in FP32) or not finite. The norms on the small
-// levels scale with d; in PCG solves of 2D Q1, 2D Q2 and 3D Q1 problems those of the levels that
-// smooth were typically above 1e-3 d (the smallest on 25 rows). So above 1024 eps^2 the test would not
-// act, or only on parts a thousand times smaller than the cycle; the upper bounds keep every sum of
-// squares finite. All other cycles run level by level, with the tests. Tiny defects are met at the end of
-// FP32 solves: the 257^3 mixed solve runs its last one or two iterations level by level, 13.71 -> 13.77
-// ms.
+// levels scale with d, in PCG solves down to about 5 d / (M / m) for M points per side of the finest level
+// and m of the smallest one that smooths. So the operator is used above 10 M / m eps^2: there one cycle on
+// the defects of such solves (2D Q1 and Q2 to 1025^2, 3D to 65^3) differed from the cycle with the tests by
+// rounding, in 4 of 24 cases by 3e-3 to 5e-3 (with twice the limit in one by 1.6e-3, with half of it in 16 by up to
+// 3e-2). The upper bounds keep every sum of squares finite. All other cycles run level by level, with the
+// tests. Defects that small are met at the end of FP32 solves: the 257^3 mixed solve runs its last iteration
+// level by level, 2D Q2 1025^2 its last one or two.
 static bool dense_applies(const fb_mg* m, double d) {
   if (m->dense_l == 0) return true;
   const bool low = m->cfg.precision != FB_PREC_F64;
   const double e = low ? double(eps_of<float>()) : eps_of<double>();
-  return d > 1024.0 * e * e && d < (low ? 3e32 : 1e148);
+  const size_t last = m->L.size() - (m->cfg.coarse == FB_COARSE_SMOOTHER ? 1 : 2);
+  const double rows = double(m->L[0].n) / double(m->L[last].n);
+  const double sides = m->dim == 3 ? std::cbrt(rows) : std::sqrt(rows);  // (a handed-over hierarchy: no less)
+  return d > 10.0 * sides * e * e && d < (low ? 3e32 : 1e148);
 }
 
 template<typename T>

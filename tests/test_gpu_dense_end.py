@@ -121,8 +121,8 @@ def test_tiny_and_non_finite_defects(case, fmt):
             ref = H.vcycle(t, nu=nu, coarse=coarse, inner=prec)  # (zero where every smoother is left out)
             assert np.linalg.norm(out - ref) <= tol * np.linalg.norm(ref), (prec, size)
         np.testing.assert_array_equal(mg.vcycle(torch.tensor(d).cuda()).cpu().numpy(), plain)
-        # iterations of a solve whose small levels meet the test
-        t = d * (900.0 * eps ** 2)
+        # iterations of a solve whose small levels meet the test (one eps^2 per point of a side)
+        t = d * (H.ndofs() ** (1.0 / dim) * eps ** 2)
         out = mg.configure(nu=nu, coarse=coarse, precision=prec, format=fmt, max_iter=2).solve(torch.tensor(t).cuda())
         ref = H.solve(t, nu=nu, coarse=coarse, inner=prec, max_iter=2)
         np.testing.assert_allclose(out["hist"], ref["hist"], rtol=1e-4 if prec == "f32" else 1e-10)

@@ -308,12 +308,12 @@ def test_unknown_flags_are_rejected():
 # Level 0 of the cycle is the finest. size: the defect's norm, or None for the right-hand side as it is.
 # With a dense small end (two or more levels of at most 1,280 rows) the cluster holds the levels above it
 # in 3D and is not used in 2D; without one it holds every level of at most 5,000 rows: where one level is
-# that small, and for defects of at most 1,024 eps^2, which leave the dense operator aside (down to
-# 27 or 9 rows here). The norms keep some of the levels inside the smoothers' skip test.
+# that small, and for defects of a few eps^2 per point of a side, which leave the dense operator aside
+# (down to 27 or 9 rows here). The norms keep some of the levels inside the smoothers' skip test.
 CLUSTER = [(dim, lvl, lmin, prec, size)
            for dim, lvl, lmin, prec in [(3, 6, 1, "f32"), (3, 5, 1, "f64"), (3, 6, 3, "f32"), (3, 5, 3, "f64"),
                                         (2, 9, 5, "f32"), (2, 8, 5, "f64"), (2, 9, 1, "f32"), (2, 8, 1, "f64")]
-           for size in (None, 500.0, 5.0) if (dim, lmin, size) != (2, 1, None)]
+           for size in (None, 50.0, 5.0) if (dim, lmin, size) != (2, 1, None)]
 
 
 @pytest.mark.parametrize("coarse", ["direct", "smoother", "none"])
