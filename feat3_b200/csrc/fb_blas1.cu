@@ -1,6 +1,6 @@
 // Vector kernels of the operator layer: axpy, dot, norm2, component product/invert,
 // scale, unit filter, precision conversion, fill. HBM-bound; grid-stride loops with
-// 16-byte vector accesses where the pointers allow it.
+// 16-byte accesses for aligned vectors beyond the L2.
 #include "fb_common.cuh"
 
 #include <cstdio>
